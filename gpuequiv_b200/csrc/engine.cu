@@ -81,7 +81,7 @@ constexpr int SM_BM2 = 128;   // 128 words: second bitmap (own / old list)
 constexpr int SM_TMP = 256;   // 32 words: segment map / compaction
 constexpr int SM_PINC = 288;  // 32 words: predecessor counts (inclusive scan)
 constexpr int SM_PBEG = 320;  // 32 words: predecessor row starts
-constexpr int SM_WORDS = 352;
+constexpr int SM_WORDS = 352; // the lane path's W_* layout uses the same words at another time
 // device error bits (Ctr::error)
 constexpr uint32_t DERR_LIST = 1u;     // a list longer than 2^24 - 1 energies
 constexpr uint32_t DERR_BOUNDS = 2u;   // checked build: index out of range
@@ -994,7 +994,7 @@ __device__ Res solve_position(const WarpCtx &x, const Cd &cd, uint32_t v) {
   else return defend_list(x, cd, e0, e1, dv);
 }
 
-// ---- thread path: one lane per small position -----------------------------
+// ---- lane path: up to 32 positions per warp, one owner lane each ------------
 // Successor and update of edge k: one 8-byte load of the edge pair, or the
 // col / wt arrays where there are none (the one-block solver).
 __device__ __forceinline__ void load_edge(const KParams &p, Ctr *c, unsigned long long k, uint32_t &w, uint32_t &u) {
@@ -1007,6 +1007,11 @@ __device__ __forceinline__ void load_edge(const KParams &p, Ctr *c, unsigned lon
     u = ld(p.wt, k, p.n_edges, c);
   }
 }
+template <class Cd>
+__device__ __forceinline__ typename Cd::Upd edge_upd(const KParams &p, const Cd &cd, uint32_t u) {
+  return p.cw ? cd.unpack_edge(u) : cd.prep(u);
+}
+
 // up to four consecutive edges k0 .. k0+min(left,4)-1
 __device__ __forceinline__ void load_edges4(const KParams &p, Ctr *c, unsigned long long k0, uint32_t left,
                                             uint32_t (&w)[4], uint32_t (&u)[4]) {
@@ -1014,11 +1019,6 @@ __device__ __forceinline__ void load_edges4(const KParams &p, Ctr *c, unsigned l
   for (int t = 0; t < 4; t++)
     if ((uint32_t)t < left) load_edge(p, c, k0 + t, w[t], u[t]);
 }
-template <class Cd>
-__device__ __forceinline__ typename Cd::Upd edge_upd(const KParams &p, const Cd &cd, uint32_t u) {
-  return p.cw ? cd.unpack_edge(u) : cd.prep(u);
-}
-
 // Most positions have a handful of successors with one or two energies each.
 // Every lane of a warp solves its own such position.  Candidates stream into
 // an antichain held in a lane-private column of shared memory (bank = lane):
@@ -1153,6 +1153,375 @@ __device__ int thread_solve(const KParams &p, Ctr *c, const Cd &cd, const uint32
   return T_CHANGED;
 }
 
+// Whether the defender fold's step over the cb codes at b leaves the antichain
+// at column words [sb, sb+ns) as it is -- most steps do.  Pairs are taken in
+// the order (code, member).  When every member has a code below it, the
+// member is its own supremum with that code and every other pair lies above a
+// member, so the result is the same set, each member placed by its first such
+// code; if those are in member order the list is unchanged.  Only asked for at
+// most TK pairs, where the full step could not have run out of room either.
+__device__ __forceinline__ bool fold_keeps(const uint32_t *scr, uint32_t sb, uint32_t ns, const uint32_t *b,
+                                           uint32_t cb) {
+  uint32_t prev = 0;
+  for (uint32_t k = 0; k < ns; k++) {
+    const uint32_t s = SCR(sb + k);
+    uint32_t q = prev;
+    while (q < cb && (b[q] & ~s) != 0u) q++;
+    if (q == cb) return false;
+    for (uint32_t f = 0; f < prev; f++)
+      if ((b[f] & ~s) == 0u) return false;  // its first code comes before its predecessor's
+    prev = q;
+  }
+  return true;
+}
+// The same step by one lane; false: beyond TK members.
+__device__ __forceinline__ bool fold_step(uint32_t *scr, uint32_t &sb, uint32_t &ns, const uint32_t *b, uint32_t cb) {
+  const uint32_t nb = sb ^ TK;
+  uint32_t nn = 0, om = 0;
+  for (uint32_t q = 0; q < cb; q++) {
+    const uint32_t bq = b[q];
+    for (uint32_t k = 0; k < ns; k++)
+      if (!ac_insert(scr, nb, nn, om, SCR(sb + k) | bq, false)) return false;
+  }
+  sb = nb;
+  ns = nn;
+  return true;
+}
+
+// ac_insert of P <= 96 candidates in turn, by the whole warp (lane l holds
+// candidates l, l+32, l+64 in c): the members left at the end are the
+// candidates without a strictly smaller one and without an equal earlier one,
+// in candidate order, since a member once minimal is never dropped.  They go
+// to col[0], col[32], ...  A serial insertion is a chain of shared-memory
+// loads and branches per pair of candidates; here a candidate meets all others
+// by shuffles that do not depend on one another.
+//
+// own: flag of candidate l (l < 32) for the tie rule; om: flags of the kept
+// members.  false where ac_insert would have found more than TK members on
+// the way: a candidate lives from its turn until the first later one strictly
+// below it.
+__device__ __forceinline__ bool warp_insert(uint32_t P, const uint32_t (&c)[3], bool own, uint32_t *col, uint32_t lane,
+                                            uint32_t &n, uint32_t &om) {
+  bool born[3] = {lane < P, lane + 32u < P, lane + 64u < P};
+  uint32_t end[3] = {~0u, ~0u, ~0u};
+#pragma unroll
+  for (int rj = 0; rj < 3; rj++) {
+    if (rj * 32u >= P) break;
+    const uint32_t nj = min(32u, P - rj * 32u);
+    for (uint32_t l = 0; l < nj; l++) {
+      const uint32_t cj = __shfl_sync(FULL, c[rj], l), j = rj * 32u + l;
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        if (r * 32u >= P) break;
+        const uint32_t i = r * 32u + lane;
+        if ((cj & ~c[r]) == 0u) {
+          if (j < i) born[r] = false;
+          else if (cj != c[r]) end[r] = min(end[r], j);
+        }
+      }
+    }
+  }
+  const uint32_t b0 = __ballot_sync(FULL, born[0]), b1 = __ballot_sync(FULL, born[1]),
+                 b2 = __ballot_sync(FULL, born[2]);
+  if ((uint32_t)(__popc(b0) + __popc(b1) + __popc(b2)) > TK) {
+    uint32_t live[3] = {0u, 0u, 0u};
+#pragma unroll
+    for (int rj = 0; rj < 3; rj++) {
+      const uint32_t bj = rj == 0 ? b0 : rj == 1 ? b1 : b2;
+      for (uint32_t m = bj; m; m &= m - 1u) {
+        const uint32_t l = (uint32_t)__ffs((int)m) - 1u, j = rj * 32u + l;
+        const uint32_t ej = __shfl_sync(FULL, end[rj], l);
+#pragma unroll
+        for (int r = 0; r < 3; r++) live[r] += j <= r * 32u + lane && ej > r * 32u + lane ? 1u : 0u;
+      }
+    }
+    if (__any_sync(FULL, (born[0] && live[0] > TK) || (born[1] && live[1] > TK) || (born[2] && live[2] > TK)))
+      return false;
+  }
+  __syncwarp();
+  uint32_t rank = 0, flags = 0;
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    if (r * 32u >= P) break;
+    const bool keep = born[r] && end[r] == ~0u;
+    const uint32_t km = __ballot_sync(FULL, keep);
+    if (keep) {
+      const uint32_t k = rank + (uint32_t)__popc(km & lanemask_lt());
+      col[k * 32u] = c[r];
+      if (r == 0 && own) flags = 1u << k;
+    }
+    rank += (uint32_t)__popc(km);
+  }
+  n = rank;
+  om = __reduce_or_sync(FULL, flags);
+  __syncwarp();
+  return true;
+}
+
+// A warp's positions, one owner lane each (the warp calls it together; `on` is
+// false for lanes without a position), for rounds whose length is the time of
+// one warp: every lane walking its own edges (thread_solve) makes that the
+// chain of dependent loads of the largest position, one list energy and one
+// antichain member after the other, while the other lanes wait.  Here the
+// edges of the warp's positions are laid end to end and
+// taken 32 at a time, one per lane: load the edge, the successor's list, apply
+// the update to each of its energies.  A candidate of an attacker that lies
+// above one of the owner's own energies is dropped on the spot (the own
+// energy, or one below it, is in the antichain when its turn comes); what is
+// left, and every updated energy of a defender, goes to the warp's buffer in
+// (position, edge, energy) order.  When the buffer is full or the edges are
+// done, each owner lane takes its range in that order: an attacker streams
+// the candidates into the antichain in its column of shared memory that starts
+// as its own list (bank = lane), a defender folds edge by edge (fold_keeps,
+// fold_step).  A step of more than COOP candidates or pairs is done for the
+// owner by the whole warp (warp_insert).
+// What remains is the set of minimal candidates, so the lists equal the
+// reference's as sets (the order inside a list may differ).  Positions beyond
+// td successors, tk members or tw candidates (per defender step: pairs) are
+// left to the warp routines (T_BIG).
+//
+// Returns T_*; with T_CHANGED the new list's out_cnt packed energies are at
+// SCR(TK) ...  ws: W_WORDS words of shared memory of the warp.
+constexpr int W_BUF = 0;      // codes of the window
+constexpr uint32_t W_BUFN = 320;
+constexpr int W_MAP = 320;    // chunk: owner of the range that starts at edge i
+constexpr int W_TOT = 352;    // per owner: energies of all successors read so far
+constexpr int W_CNT = 384;    // per owner: codes in the window
+constexpr int W_EC = 416;     // per edge of the window: its codes (bytes)
+constexpr uint32_t W_EDGES = 256;
+constexpr int W_WORDS = 480;
+constexpr uint32_t COOP = 8;      // defender steps of more pairs are done by the warp
+constexpr uint32_t COOP_ATT = 4;  // attackers with more codes in the window
+// Frontiers of at most this many slots per warp of the grid are spread over
+// all warps (lanes_solve), a warp of larger ones takes 32 slots at a time
+// (thread_solve).
+constexpr uint32_t SPREAD_SLOTS = 16;
+constexpr uint32_t SPREAD_MIN = 2;  // slots a warp takes at least
+
+template <class Cd>
+__device__ __forceinline__ int lanes_solve(const KParams &p, Ctr *c, const Cd &cd, const uint32_t *arena,
+                                           unsigned long long cap, uint32_t v, bool on, uint32_t *ws, uint32_t *scr,
+                                           uint32_t lane, uint32_t &out_cnt, uint32_t &edges, uint32_t &bytes,
+                                           uint32_t &old_cnt) {
+  int ts = T_NONE;
+  uint32_t e0 = 0, d = 0, cv = 0;
+  unsigned long long dv = 0;
+  bool att = false;
+  if (on) {
+    e0 = ld(p.row, v, p.n_nodes + 1, c);
+    d = ld(p.row, (unsigned long long)v + 1, p.n_nodes + 1, c) - e0;
+    ts = d == 0 ? T_SKIPPED : (!p.thread_path || d > p.td) ? T_BIG : T_NONE;
+    if (ts == T_NONE) {
+      dv = ld(p.desc, v, p.n_nodes, c);
+      cv = dcnt(dv);
+      att = ld(p.flags, v, p.n_nodes, c) & 1u;
+      old_cnt = cv;
+      if (att && cv > p.tk) ts = T_BIG;
+    }
+  }
+  // n: members of the attacker's antichain / the defender's running list
+  uint32_t n = 0, om = 0, sb = 0;
+  bool big = false;
+  const bool mine = on && ts == T_NONE;
+  if (mine && att) {
+    // the own energies first (the old minimal set, all flagged own); a
+    // candidate equal to an own member is dropped, so the own copy stays (the
+    // later copy wins, attack_minimize.wgsl:84-92)
+    for (uint32_t q = 0; q < cv && !big; q++)
+      big = !ac_insert(scr, 0, n, om, cd.to_t(lelem(dv, q, arena, cap, c, p.ib, p.ibm)), true);
+  }
+  const uint32_t dl = mine && !big ? d : 0u;
+  const uint32_t incl = warp_incl_scan(dl, lane), excl = incl - dl;
+  const uint32_t E = __shfl_sync(FULL, incl, 31);
+  ws[W_TOT + lane] = 0u;
+  uint32_t *scr0 = scr - lane;
+  uint8_t *ec = (uint8_t *)(ws + W_EC);
+  uint32_t empty = 0u, bigm = __ballot_sync(FULL, big);  // owners with an empty successor / to leave to a warp
+  // an owner's word for its edges: edge id - position in the concatenation,
+  // and kind, single edge, own members in one word
+  const uint32_t ebase = e0 - excl;
+  const uint32_t oinfo = n | (att ? 32u : 0u) | (d == 1u ? 64u : 0u);
+  uint32_t w0 = 0;
+  while (w0 < E) {
+    ws[W_CNT + lane] = 0u;
+    uint32_t used = 0, t = w0;
+    while (t < E && t - w0 <= W_EDGES - 32u) {
+      // owners whose edges fall into [t, t+32)
+      const bool in = dl != 0u && incl > t && excl < t + 32u;
+      const uint32_t at = excl > t ? excl - t : 0u;
+      const uint32_t heads = __reduce_or_sync(FULL, in ? 1u << at : 0u);
+      __syncwarp();
+      if (in) ws[W_MAP + at] = lane;
+      __syncwarp();
+      const uint32_t k = t + lane;
+      const bool has = k < E;
+      const uint32_t o = ws[W_MAP + (31u - (uint32_t)__clz((int)(heads & (2u * (1u << lane) - 1u))))] & 31u;
+      const uint32_t eb = __shfl_sync(FULL, ebase, o), oi = __shfl_sync(FULL, oinfo, o);
+      uint32_t cnt = 0, u = 0;
+      unsigned long long dw = 0;
+      if (has) {
+        uint32_t w = 0;
+        load_edge(p, c, (unsigned long long)(eb + k), w, u);
+        dw = ld(p.desc, w, p.n_nodes, c);
+        cnt = dcnt(dw);
+      }
+      const bool oatt = (oi & 32u) != 0u;
+      const bool none = has && cnt == 0u && !oatt;
+      const bool many = has && cnt > ((oi & 96u) == 64u ? p.tk : p.tw);
+      if (__any_sync(FULL, none)) empty |= __reduce_or_sync(FULL, none ? 1u << o : 0u);
+      if (__any_sync(FULL, many)) bigm |= __reduce_or_sync(FULL, many ? 1u << o : 0u);
+      if (many) cnt = 0u;
+      const auto pu = edge_upd(p, cd, u);
+      // survivors of an attacker's edge (the first 32 energies are tested)
+      uint32_t nl = cnt, surv = 0u;
+      if (oatt) {
+        const uint32_t on_ = oi & 31u, ct = min(cnt, 32u);
+        for (uint32_t q = 0; q < ct; q++) {
+          const uint32_t x = cd.apply(cd.to_t(lelem(dw, q, arena, cap, c, p.ib, p.ibm)), pu);
+          bool dom = false;
+          for (uint32_t m = 0; m < on_; m++) dom |= (scr0[m * 32u + o] & ~x) == 0u;
+          if (!dom) surv |= 1u << q;
+        }
+        nl = (uint32_t)__popc(surv) + (cnt - ct);
+      }
+      const uint32_t ci = warp_incl_scan(nl, lane);
+      const bool acc = has && used + ci <= W_BUFN;
+      const uint32_t accm = __ballot_sync(FULL, acc);  // a prefix of the lanes
+      if (acc) {
+        if (cnt) atomicAdd(&ws[W_TOT + o], cnt);
+        uint32_t to = W_BUF + used + ci - nl;
+        if (oatt) {
+          while (surv) {
+            const uint32_t q = (uint32_t)__ffs((int)surv) - 1u;
+            surv &= surv - 1u;
+            ws[to++] = cd.apply(cd.to_t(lelem(dw, q, arena, cap, c, p.ib, p.ibm)), pu);
+          }
+          for (uint32_t q = 32u; q < cnt; q++)
+            ws[to++] = cd.apply(cd.to_t(lelem(dw, q, arena, cap, c, p.ib, p.ibm)), pu);
+        } else {
+          for (uint32_t q = 0; q < cnt; q++)
+            ws[to++] = cd.apply(cd.to_t(lelem(dw, q, arena, cap, c, p.ib, p.ibm)), pu);
+          ec[k - w0] = (uint8_t)nl;
+        }
+        if (nl) atomicAdd(&ws[W_CNT + o], nl);
+      }
+      const uint32_t na = (uint32_t)__popc(accm);
+      if (na) used += __shfl_sync(FULL, ci, na - 1u);
+      t += na;
+      if (na < min(32u, E - (t - na))) break;  // the buffer is full
+    }
+    __syncwarp();
+    // the owners take their codes
+    uint32_t mc = ws[W_CNT + lane];
+    uint32_t off = W_BUF + warp_incl_scan(mc, lane) - mc;
+    const bool act = dl && !(((empty | bigm) >> lane) & 1u);
+    uint32_t k = max(excl, w0);
+    const uint32_t ke = act && !att ? min(incl, t) : 0u;
+    if (!act || !att) mc = 0u;
+    for (;;) {
+      // P: candidates of the owner's next step when it is one for the warp
+      uint32_t P = 0, cb = 0;
+      if (mc) {
+        if (mc > TW) big = true;  // more than tw energies
+        else if (mc > COOP_ATT) P = n + mc;
+        else
+          for (uint32_t i = 0; i < mc && !big; i++) big = !ac_insert(scr, 0, n, om, ws[off + i], false);
+        if (!P) mc = 0u;
+      }
+      // d == 1: the successor's updated list as is
+      // (defend_iterative.wgsl:200-211); else the fold of pairwise suprema,
+      // minimised after every step (defend_iterative.wgsl:215-262) -- the
+      // first list minimised too, which leaves the minimal suprema unchanged
+      while (k < ke && !big) {
+        cb = ec[k - w0];
+        if (k == excl) {
+          if (d == 1u) {
+            for (uint32_t q = 0; q < cb; q++) SCR(q) = ws[off + q];
+            n = cb;
+          } else if (cb > COOP) {
+            P = cb;
+            break;
+          } else {
+            for (uint32_t q = 0; q < cb && !big; q++) big = !ac_insert(scr, 0, n, om, ws[off + q], false);
+          }
+        } else {
+          const uint32_t pairs = n * cb;
+          if (pairs > p.tw) {
+            big = true;
+          } else if (pairs > TK || !fold_keeps(scr, sb, n, ws + off, cb)) {
+            if (pairs > COOP) {
+              P = pairs;
+              break;
+            }
+            big = !fold_step(scr, sb, n, ws + off, cb);
+          }
+        }
+        off += cb;
+        k++;
+      }
+      uint32_t hm = __ballot_sync(FULL, P != 0u);
+      if (!hm) break;
+      __syncwarp();
+      for (; hm; hm &= hm - 1u) {
+        const uint32_t L = (uint32_t)__ffs((int)hm) - 1u;
+        const uint32_t lP = __shfl_sync(FULL, P, L), ln = __shfl_sync(FULL, n, L), loff = __shfl_sync(FULL, off, L),
+                       lsb = __shfl_sync(FULL, sb, L), lom = __shfl_sync(FULL, om, L);
+        // 0: an attacker's members, then its codes; 1: codes; 2: members x codes
+        const uint32_t kind = __shfl_sync(FULL, att ? 0u : k == excl ? 1u : 2u, L);
+        uint32_t *col = scr0 + lsb * 32u + L;
+        uint32_t cc[3] = {0u, 0u, 0u};
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          const uint32_t i = r * 32u + lane;
+          if (i < lP) {
+            if (kind == 0u) cc[r] = i < ln ? col[i * 32u] : ws[loff + i - ln];
+            else if (kind == 1u) cc[r] = ws[loff + i];
+            else cc[r] = col[(i % ln) * 32u] | ws[loff + i / ln];
+          }
+        }
+        uint32_t nn = 0, no = 0;
+        const bool ok = warp_insert(lP, cc, kind == 0u && lane < ln && ((lom >> lane) & 1u), col, lane, nn, no);
+        if (lane == L) {
+          big = !ok;
+          n = ok ? nn : n;
+          om = no;
+          mc = 0u;
+          off += cb;
+          k++;
+        }
+      }
+    }
+    bigm |= __ballot_sync(FULL, big);
+    w0 = t;
+    __syncwarp();
+  }
+  if (!mine) return ts;
+  const uint32_t tot = ws[W_TOT + lane];
+  // defender: skipped while a successor has no energies (energygame.rs:789-792)
+  if ((empty >> lane) & 1u) return T_SKIPPED;
+  if (((bigm >> lane) & 1u) || (att && tot > p.tw)) return T_BIG;
+  edges += d;
+  bytes += 12u + 16u * d + 4u * tot;
+  if (att) {
+    bytes += 4u * cv;
+    if (om == (1u << n) - 1u) return T_UNCHANGED;
+  }
+  for (uint32_t q = 0; q < n; q++) SCR(TK + q) = cd.to_p(SCR(sb + q));
+  if (!att) {
+    // EnergyArray PartialEq (energy.rs:334-350) against the old list
+    bool changed = n != cv;
+    for (uint32_t i = 0; i < n && !changed; i++) {
+      const uint32_t x = SCR(TK + i);
+      bool found = false;
+      for (uint32_t j = 0; j < cv && !found; j++) found = lelem(dv, j, arena, cap, c, p.ib, p.ibm) == x;
+      changed = !found;
+    }
+    if (!changed) return T_UNCHANGED;
+  }
+  out_cnt = n;
+  return T_CHANGED;
+}
+
 // The next frontier is a bitmap: one bit per position in each of two halves
 // of `mark`, chosen by the parity of the stamp of the round that pushes.
 // After the round k_commit counts the half's bits per block and clears the
@@ -1217,7 +1586,7 @@ __device__ void push_preds_warp(const KParams &p, Ctr *c, uint32_t *sm, uint32_t
 
 template <class Cd, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) k_round(const KParams p) {
-  __shared__ uint32_t smem[WARPS_PER_BLOCK * SM_WORDS];
+  __shared__ uint32_t smem[WARPS_PER_BLOCK * W_WORDS];
   __shared__ uint32_t tscr[WARPS_PER_BLOCK * TSCR * 32];
   Ctr *c = p.ctr;
   if (c->halt) return;
@@ -1227,34 +1596,49 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_round(const KParams p) {
   const uint32_t *F = cur ? p.front1 : p.front0;
   const uint32_t stamp = c->stamp + 1u;
   const uint32_t lane = threadIdx.x & 31u;
-  uint32_t *sm = smem + (threadIdx.x >> 5) * SM_WORDS;
+  uint32_t *sm = smem + (threadIdx.x >> 5) * W_WORDS;
   uint32_t *scr = tscr + (threadIdx.x >> 5) * (TSCR * 32) + lane;
   const Cd cd = make_codec<Cd>(p);
   uint32_t *arena = c->arena;
   const unsigned long long cap = c->arena_cap;
   WarpAlloc wa{0, 0};
+  const uint32_t nwarps = gridDim.x * WARPS_PER_BLOCK;
+  // A small round is as long as its slowest warp: its positions are spread
+  // over all warps, each of which works on a few of them together.  Measured
+  // on one B200 (4 blocks per SM: 4,736 warps), median per round of the last
+  // 28 of 48 rounds (fewer than 75,000 slots) of 1,400 spectroscopy games:
+  // 95 us with thread_solve, 24 us with lanes_solve; a 42,000-position game's
+  // 16 rounds: 541 -> 302 us; 2M-position bipartite game: 1.56 -> 1.21 ms.  In
+  // a large round every warp is busy anyway and thread_solve issues fewer
+  // instructions per position (rounds of over 300,000 slots: 0.43-1.17 ms
+  // against 0.48-1.23 ms with lanes_solve); the line at 8 or 16 slots per warp
+  // gave the same solve time.
+  const bool spread = fs <= SPREAD_SLOTS * nwarps;
+  const uint32_t grab = spread ? max(SPREAD_MIN, (fs + nwarps - 1u) / nwarps) : 32u;
   uint32_t t_edges = 0, t_bytes = 0, t_pos = 0;  // per lane, this launch
 #if GEQ_PATH_PROFILE
   unsigned long long prof_acc[16] = {};
   const long long t_all0 = clock64();
 #endif
   for (;;) {
-    // 32 slots at a time from a shared counter: warps that drew heavy
-    // positions take fewer slots
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(&c->next_slot, 32u);
+    if (lane == 0) base = atomicAdd(&c->next_slot, grab);
     base = __shfl_sync(FULL, base, 0);
     if (base >= fs) break;
 #if GEQ_PATH_PROFILE
     const long long tq0 = clock64();
 #endif
     const uint32_t slot = base + lane;
-    const bool active = slot < fs;
+    const bool active = lane < grab && slot < fs;
     const uint32_t v = active ? ld(F, slot, p.n_nodes, c) : 0u;
-    int ts = T_NONE;
     uint32_t cnt = 0, old_cnt = 0;
-    if (active)
-      ts = p.thread_path ? thread_solve(p, c, cd, arena, cap, v, scr, cnt, t_edges, t_bytes, old_cnt) : T_BIG;
+    int ts = T_NONE;
+    if (!spread) {
+      if (active)
+        ts = p.thread_path ? thread_solve(p, c, cd, arena, cap, v, scr, cnt, t_edges, t_bytes, old_cnt) : T_BIG;
+    } else {
+      ts = lanes_solve(p, c, cd, arena, cap, v, active, sm, scr, lane, cnt, t_edges, t_bytes, old_cnt);
+    }
     if (ts != T_NONE && ts != T_BIG && ts != T_SKIPPED) t_pos++;
     // inline results need no arena; one reservation for the others
     unsigned long long nd = NONE_DESC;
