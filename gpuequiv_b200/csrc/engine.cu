@@ -39,6 +39,7 @@
 // lists are the minimal elements of that fixpoint, and a single-successor
 // defender's list is the image of its successor's list.
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -2513,6 +2514,27 @@ void HostBuf::reset() {
   pool.reset();
 }
 
+// Where rounds run inside one launch (k_rounds_cluster, k_solve_static), on one
+// B200, each figure the median of whole calls:
+// - uploads of up to CLUSTER_POSITIONS run all their rounds in cluster
+//   launches: stress games of 20,000 positions 457 -> 318 us; with the line at
+//   65,536, spectroscopy games of 42,000 and 60,000 positions 1,060 -> 1,250
+//   and 1,180 -> 1,420 us (16 blocks are too few for their middle rounds);
+// - larger ones, up to CLUSTER_POSITIONS_TAIL (every block counts the whole
+//   bitmap, 128 KB there), from the step on that leaves at most
+//   CLUSTER_FRONTIER positions (1,024 to 4,096: the same within noise);
+// - a lone game of up to SMALL_GAME_POSITIONS is one launch from input to
+//   result: 2,500 positions 578 -> 162 us (one block of 8 warps before),
+//   9,000: 736 -> 280 us, 30,000: 720 -> 663 us (upload and graphs of rounds
+//   before);
+// - of those, up to STATIC_ONE_BLOCK by one block, whose barrier is cheaper
+//   than a cluster's (300 positions: 105 against 126 us; 800: 129 against
+//   124), of 8 warps up to STATIC_FEW_WARPS (80 positions: 66 us, 74 with 16).
+constexpr unsigned long long CLUSTER_POSITIONS = 32768, CLUSTER_POSITIONS_TAIL = 1ull << 20;
+constexpr uint32_t CLUSTER_FRONTIER = 2048;
+constexpr uint32_t CLUSTER_ROUNDS = 256, CLUSTER_ROUNDS_SERVING = 16;  // per launch
+constexpr unsigned long long STATIC_ONE_BLOCK = 400, STATIC_FEW_WARPS = 256;
+
 struct Engine::State {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, eva = nullptr, evb = nullptr;
@@ -2521,7 +2543,8 @@ struct Engine::State {
   // uploads; its kernel nodes get the parameters of the games being solved
   cudaGraph_t graph[2] = {nullptr, nullptr};
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  std::vector<cudaGraphNode_t> gnodes[2];
+  std::vector<cudaGraphNode_t> gnodes[2];  // four per round, in launch order
+  uint32_t cluster = 1;  // blocks of the cluster kernels: 16 where the device takes it, else 8
   uint32_t g_rounds[2] = {0, 0}, g_bps[2] = {0, 0};
   KParams g_kp[2] = {};              // the parameters the graph's nodes hold
   bool g_kp_valid[2] = {false, false};
@@ -2572,6 +2595,7 @@ struct DeviceGamesImpl {
     double round_ms = 0.0;
     std::chrono::steady_clock::time_point t_start{};
   } prog;
+  uint32_t frontier = ~0u;  // its size after the last step (unknown before the first)
   HostBuf hstep;            // page-locked: the control block and active flags read back by a step
   uint8_t *d_act = nullptr; // active flags on the device
   bool step_active = false;
@@ -2739,6 +2763,9 @@ void *Engine::stream_handle() const { return (void *)st->stream; }
 std::shared_ptr<HostPool> Engine::host_pool() const { return st->hpool; }
 
 static geq_status static_scratch(int device, unsigned char *&out);
+static geq_status cluster_setup(uint32_t &blocks);
+static geq_status launch_rounds_cluster(const Engine &E, const KParams &kp, bool generic, uint32_t max_rounds,
+                                        uint32_t limit);
 
 geq_status Engine::create(int device, std::unique_ptr<Engine> &out) {
   int n = 0;
@@ -2779,6 +2806,10 @@ geq_status Engine::create(int device, std::unique_ptr<Engine> &out) {
   CU(cudaFuncSetAttribute(k_round<CodecGen, 5>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   CU(cudaFuncSetAttribute(k_round_big<CodecStd>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   CU(cudaFuncSetAttribute(k_round_big<CodecGen>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  {
+    const geq_status cs = cluster_setup(s.cluster);
+    if (cs) return cs;
+  }
   int bps = 0;
   CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_round<CodecStd, 4>, BLOCK, 0));
   eng->tuning.blocks_per_sm = (uint32_t)std::max(2, std::min(bps, 4));
@@ -3211,7 +3242,10 @@ geq_status Engine::finish_upload(GamesPtr &dg, bool any_init, GamesPtr &out) {
   kp.slot_new = D.slot_new; kp.ctr = D.ctr; kp.n_nodes = N; kp.n_edges = M;
   kp.mwords = (uint32_t)((N + 31) / 32);
   kp.fpart = D.fpart;
-  kp.fblocks = (uint32_t)std::max(1, n_sms * GEQ_FRONTIER_BLOCKS_PER_SM);
+  // a block per 512 positions (16 words of the bitmap) at most: the launch of
+  // more blocks than a small upload has work for is what its rounds would wait for
+  kp.fblocks = (uint32_t)std::max<unsigned long long>(
+      1, std::min<unsigned long long>((unsigned long long)n_sms * GEQ_FRONTIER_BLOCKS_PER_SM, (N + 511) / 512));
   kp.abits = D.abits;
   kp.bigq = D.bigq;
   kp.cw = D.cw;
@@ -3269,67 +3303,91 @@ static void set_lane_limits(KParams &kp, const geq_tuning &t) {
   kp.tk = k ? std::min(k, TK) : TK;
 }
 
+// The four kernels of a round and their grids: as many blocks as the upload
+// can have work for (SPREAD_MIN slots per warp of k_round, a warp per large
+// position of k_round_big), at most those resident at once.  Measured on one
+// B200: an idle k_round_big of 592 blocks takes 5.7 us, of 8 blocks 1.5 us.
+struct RoundKernel {
+  void *f;
+  dim3 grid, block;
+};
 template <class Cd>
-static void launch_round(Engine &E, const KParams &kp, cudaStream_t S, cudaEvent_t ea = nullptr,
-                         cudaEvent_t eb = nullptr) {
+static void round_kernels(const Engine &E, const KParams &kp, RoundKernel (&k)[4]) {
   const uint32_t bps = std::min<uint32_t>(std::max<uint32_t>(E.tuning.blocks_per_sm, 2), 5);
-  const unsigned grid = (unsigned)std::max<uint32_t>(1, E.n_sms * bps);
-  if (ea) cudaEventRecord(ea, S);
-  if (bps == 2) k_round<Cd, 2><<<grid, BLOCK, 0, S>>>(kp);
-  else if (bps == 3) k_round<Cd, 3><<<grid, BLOCK, 0, S>>>(kp);
-  else if (bps == 4) k_round<Cd, 4><<<grid, BLOCK, 0, S>>>(kp);
-  else k_round<Cd, 5><<<grid, BLOCK, 0, S>>>(kp);
-  k_round_big<Cd><<<(unsigned)std::max(1, E.n_sms * GEQ_BIG_BLOCKS_PER_SM), BLOCK, 0, S>>>(kp);
-  if (eb) cudaEventRecord(eb, S);
-  k_commit<<<kp.fblocks, 256, 0, S>>>(kp);
-  k_ffill<<<kp.fblocks, 256, 0, S>>>(kp);
+  const unsigned long long nr = (kp.n_nodes + WARPS_PER_BLOCK * SPREAD_MIN - 1) / (WARPS_PER_BLOCK * SPREAD_MIN),
+                           nb = (kp.n_nodes + WARPS_PER_BLOCK - 1) / WARPS_PER_BLOCK;
+  auto clamp = [](unsigned long long n, unsigned long long most) {
+    return dim3((unsigned)std::max<unsigned long long>(1, std::min(n, most)));
+  };
+  k[0].f = bps == 2 ? (void *)k_round<Cd, 2> : bps == 3 ? (void *)k_round<Cd, 3> : bps == 4 ? (void *)k_round<Cd, 4>
+                                                                                           : (void *)k_round<Cd, 5>;
+  k[0].grid = clamp(nr, (unsigned long long)E.n_sms * bps);
+  k[1].f = (void *)k_round_big<Cd>;
+  k[1].grid = clamp(nb, (unsigned long long)E.n_sms * GEQ_BIG_BLOCKS_PER_SM);
+  k[2].f = (void *)k_commit;
+  k[3].f = (void *)k_ffill;
+  k[2].grid = k[3].grid = dim3(kp.fblocks);
+  for (auto &x : k) x.block = dim3(256);
+  static_assert(BLOCK == 256, "the frontier kernels run 256 threads");
+}
+static void round_kernels(const Engine &E, const KParams &kp, bool generic, RoundKernel (&k)[4]) {
+  if (generic) round_kernels<CodecGen>(E, kp, k);
+  else round_kernels<CodecStd>(E, kp, k);
 }
 
-// One captured graph of R rounds per codec, shared by every upload: before a
-// solve its kernel nodes are pointed at the parameters of that upload.
+static geq_status launch_round(Engine &E, const KParams &kp, bool generic, cudaStream_t S, cudaEvent_t ea = nullptr,
+                               cudaEvent_t eb = nullptr) {
+  RoundKernel k[4];
+  round_kernels(E, kp, generic, k);
+  void *args[1] = {(void *)&kp};
+  if (ea) CU(cudaEventRecord(ea, S));
+  for (int i = 0; i < 4; i++) {
+    CU(cudaLaunchKernel(k[i].f, k[i].grid, k[i].block, args, 0, S));
+    if (i == 1 && eb) CU(cudaEventRecord(eb, S));
+  }
+  return GEQ_OK;
+}
+
+// One graph of R rounds per codec, shared by every upload: before a solve its
+// kernel nodes are pointed at the parameters and grids of that upload.
 static geq_status round_graph(Engine &E, const KParams &kp, bool generic, uint32_t R, cudaGraphExec_t &out) {
   Engine::State &s = *E.st;
   const int k = generic ? 1 : 0;
+  RoundKernel rk[4];
+  round_kernels(E, kp, generic, rk);
+  void *args[1] = {(void *)&kp};
+  cudaKernelNodeParams np[4] = {};
+  for (int i = 0; i < 4; i++) {
+    np[i].func = rk[i].f;
+    np[i].gridDim = rk[i].grid;
+    np[i].blockDim = rk[i].block;
+    np[i].kernelParams = args;
+  }
   if (!(s.gexec[k] && s.g_rounds[k] == R && s.g_bps[k] == E.tuning.blocks_per_sm)) {
     if (s.gexec[k]) { cudaGraphExecDestroy(s.gexec[k]); s.gexec[k] = nullptr; }
     if (s.graph[k]) { cudaGraphDestroy(s.graph[k]); s.graph[k] = nullptr; }
-    cudaStream_t cs;
-    CU(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    cudaError_t ce = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-    if (ce == cudaSuccess) {
-      for (uint32_t r = 0; r < R; r++) {
-        if (generic) launch_round<CodecGen>(E, kp, cs);
-        else launch_round<CodecStd>(E, kp, cs);
-      }
-      ce = cudaStreamEndCapture(cs, &s.graph[k]);
+    s.gnodes[k].clear();
+    s.g_kp_valid[k] = false;
+    cudaError_t ce = cudaGraphCreate(&s.graph[k], 0);
+    for (uint32_t i = 0; i < 4 * R && ce == cudaSuccess; i++) {
+      cudaGraphNode_t n = nullptr;
+      ce = cudaGraphAddKernelNode(&n, s.graph[k], i ? &s.gnodes[k].back() : nullptr, i ? 1 : 0, &np[i & 3]);
+      if (ce == cudaSuccess) s.gnodes[k].push_back(n);
     }
-    cudaStreamDestroy(cs);
     if (ce == cudaSuccess) ce = cudaGraphInstantiate(&s.gexec[k], s.graph[k], 0);
-    size_t n = 0;
-    if (ce == cudaSuccess) ce = cudaGraphGetNodes(s.graph[k], nullptr, &n);
-    s.gnodes[k].assign(n, nullptr);
-    if (ce == cudaSuccess && n) ce = cudaGraphGetNodes(s.graph[k], s.gnodes[k].data(), &n);
-    if (ce != cudaSuccess) return fail(GEQ_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
+    if (ce != cudaSuccess) {
+      s.gexec[k] = nullptr;
+      return fail(GEQ_ERR_CUDA, "round graph: %s", cudaGetErrorString(ce));
+    }
     s.g_rounds[k] = R;
     s.g_bps[k] = E.tuning.blocks_per_sm;
-    s.g_kp[k] = kp;
-    s.g_kp_valid[k] = true;
   } else if (!(s.g_kp_valid[k] && std::memcmp(&s.g_kp[k], &kp, sizeof(KParams)) == 0)) {
     s.g_kp_valid[k] = false;
-    for (cudaGraphNode_t node : s.gnodes[k]) {
-      cudaGraphNodeType t;
-      CU(cudaGraphNodeGetType(node, &t));
-      if (t != cudaGraphNodeTypeKernel) continue;
-      cudaKernelNodeParams np;
-      CU(cudaGraphKernelNodeGetParams(node, &np));
-      void *args[1] = {(void *)&kp};
-      np.kernelParams = args;
-      np.extra = nullptr;
-      CU(cudaGraphExecKernelNodeSetParams(s.gexec[k], node, &np));
-    }
-    s.g_kp[k] = kp;
-    s.g_kp_valid[k] = true;
+    for (size_t i = 0; i < s.gnodes[k].size(); i++)
+      CU(cudaGraphExecKernelNodeSetParams(s.gexec[k], s.gnodes[k][i], &np[i & 3]));
   }
+  s.g_kp[k] = kp;
+  s.g_kp_valid[k] = true;
   out = s.gexec[k];
   return GEQ_OK;
 }
@@ -3346,6 +3404,7 @@ geq_status Engine::solve_begin(DeviceGamesImpl &dg) {
   DeviceGamesImpl::Progress &pr = dg.prog;
   pr = DeviceGamesImpl::Progress{};
   pr.t_start = std::chrono::steady_clock::now();
+  dg.frontier = ~0u;
   // restart from the uploaded initial state
   const int a0 = dg.arena_cur;
   CU(cudaEventRecord(s.ev0, S));
@@ -3520,7 +3579,16 @@ geq_status Engine::step_enqueue(DeviceGamesImpl &dg, bool active) {
   const uint32_t R = use_graph ? std::max<uint32_t>(1, tuning.rounds_per_graph) : 1;
   const size_t hbytes = sizeof(Ctr) + dg.n_games;
   if (!dg.hstep.p && !dg.hstep.alloc(s.hpool, hbytes)) return fail(GEQ_ERR_OUT_OF_MEMORY, "step read-back");
-  if (use_graph) {
+  // small uploads, and the rounds of medium ones whose frontier has become
+  // small, run inside one launch of a cluster of blocks
+  const bool whole = dg.N <= CLUSTER_POSITIONS;
+  const bool cluster = use_graph && (whole || (dg.N <= CLUSTER_POSITIONS_TAIL && dg.frontier <= CLUSTER_FRONTIER));
+  if (cluster) {
+    geq_status g = launch_rounds_cluster(*this, dg.kp, dg.generic, active ? CLUSTER_ROUNDS_SERVING : CLUSTER_ROUNDS,
+                                         whole ? ~0u : 2 * CLUSTER_FRONTIER);
+    if (g) return g;
+    pr.launches++;
+  } else if (use_graph) {
     // the shared graph is pointed at this upload's parameters when they differ
     cudaGraphExec_t gexec = nullptr;
     geq_status g = round_graph(*this, dg.kp, dg.generic, R, gexec);
@@ -3528,10 +3596,10 @@ geq_status Engine::step_enqueue(DeviceGamesImpl &dg, bool active) {
     CU(cudaGraphLaunch(gexec, S));
   } else {
     cudaEvent_t ea = profile ? s.eva : nullptr, eb = profile ? s.evb : nullptr;
-    if (dg.generic) launch_round<CodecGen>(*this, dg.kp, S, ea, eb);
-    else launch_round<CodecStd>(*this, dg.kp, S, ea, eb);
+    geq_status g = launch_round(*this, dg.kp, dg.generic, S, ea, eb);
+    if (g) return g;
   }
-  pr.launches += 4ull * R;
+  if (!cluster) pr.launches += 4ull * R;
   CU(cudaMemcpyAsync(dg.hstep.p, dg.ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, S));
   dg.step_active = active && dg.n_games > 0;
   if (dg.step_active) {
@@ -3568,6 +3636,7 @@ geq_status Engine::step_finish(DeviceGamesImpl &dg, bool &done, const uint8_t *&
     pr.compactions++;
     if (c.overflow) return GEQ_OK;  // the halted rounds run at the next step; nothing retires now
   }
+  dg.frontier = c.fsize[c.cur];
   if (c.fsize[c.cur] == 0) {
     done = true;
     dg.next_stamp = c.stamp + 2u;
@@ -3951,150 +4020,127 @@ struct StaticArgs {
   uint32_t *arena;
   unsigned long long arena_cap;  // words
   unsigned long long *out_off;   // n_nodes + 1 result offsets
+  // page-locked host memory the kernel reads and writes itself (null: the host
+  // copies): the staged game, copied to `dst` first; the control block, the
+  // offsets and, when they fit in h_cap words, the energies at the end.  For
+  // a game of a few hundred positions each copy and each wait between the
+  // copies costs as much as the kernel's rounds.
+  const uint4 *h_in;
+  uint4 *dst;
+  unsigned long long in_vecs;
+  Ctr *h_ctr;
+  unsigned long long *h_off;
+  uint32_t *h_data;
+  unsigned long long h_cap;
 };
-// Games up to these sizes take the one-block path in geq_energy_game_run.
-constexpr unsigned long long SMALL_GAME_POSITIONS = 4096, SMALL_GAME_EDGES = 65536;
+// Games up to these sizes take the one-launch path in geq_energy_game_run.
+constexpr unsigned long long SMALL_GAME_POSITIONS = 32768, SMALL_GAME_EDGES = 8 * SMALL_GAME_POSITIONS;
 // Ctr::pad bits of the static solve
 constexpr uint32_t SERR_COL = 1u, SERR_WEIGHT = 2u, SERR_ARENA = 4u, SERR_ROUNDS = 8u;
 
-// out[v] = sum of cnt(u) for u < v, out[n] = the total; one block.
-template <class T, class F>
-__device__ void block_excl_scan_n(unsigned long long n, F cnt, T *out, unsigned long long *ws) {
-  const uint32_t t = threadIdx.x;
-  const unsigned long long chunk = (n + BLOCK - 1) / BLOCK;
-  const unsigned long long b = min(n, (unsigned long long)t * chunk), e = min(n, b + chunk);
-  unsigned long long sum = 0;
-  for (unsigned long long v = b; v < e; v++) sum += cnt(v);
-  ws[t] = sum;
-  __syncthreads();
-  if (t == 0) {
-    unsigned long long acc = 0;
-    for (int i = 0; i < BLOCK; i++) {
-      const unsigned long long x = ws[i];
-      ws[i] = acc;
-      acc += x;
-    }
-    out[n] = (T)acc;
+// ---- rounds inside one launch ------------------------------------------------
+// A cluster of blocks (or one block) that runs rounds without leaving the
+// kernel: a round of four kernels costs their launches and drains, which for
+// a frontier of a few thousand positions is most of the round.  Barriers are
+// the cluster's hardware barrier, so nothing spins.  The round's state (which
+// frontier list, its size, the stamp) is kept by every block alike: each block
+// counts the whole bitmap itself and writes its own slice of the next list.
+namespace cg = cooperative_groups;
+constexpr uint32_t CW = 16;             // warps per block at most
+constexpr uint32_t CT = 32 * CW;        // threads
+constexpr uint32_t CWARP_WORDS = W_WORDS + TSCR * 32;  // shared memory of a warp
+constexpr size_t cluster_smem(uint32_t warps) { return (size_t)warps * CWARP_WORDS * 4; }
+
+struct Group {
+  uint32_t rank, blocks;  // this block in its cluster
+  uint32_t tid, threads;  // this thread in the cluster
+  __device__ __forceinline__ void sync() const {
+    if (blocks > 1u) cg::this_cluster().sync();
+    else __syncthreads();
+  }
+};
+__device__ __forceinline__ Group this_group() {
+  const cg::cluster_group cl = cg::this_cluster();
+  Group g;
+  g.rank = cl.block_rank();
+  g.blocks = cl.num_blocks();
+  g.tid = g.rank * blockDim.x + threadIdx.x;
+  g.threads = g.blocks * blockDim.x;
+  return g;
+}
+
+struct RoundState {
+  uint32_t cur, fs, stamp, rounds;
+};
+
+// Words [0, words) of the bitmap: all set bits and those before word `upto`,
+// summed over the block (every thread gets both).
+__device__ __forceinline__ void block_count_bits(const uint32_t *mh, uint32_t words, uint32_t upto, uint32_t *wsum,
+                                                 uint32_t &all, uint32_t &before) {
+  uint32_t a = 0, b = 0;
+  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) {
+    const uint32_t k = (uint32_t)__popc(mh[i]);
+    a += k;
+    if (i < upto) b += k;
+  }
+  a = __reduce_add_sync(FULL, a);
+  b = __reduce_add_sync(FULL, b);
+  const uint32_t warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31u) == 0u) {
+    wsum[warp] = a;
+    wsum[CW + warp] = b;
   }
   __syncthreads();
-  unsigned long long acc = ws[t];
-  for (unsigned long long v = b; v < e; v++) {
-    out[v] = (T)acc;
-    acc += cnt(v);
+  all = before = 0;
+  for (uint32_t w = 0; w < blockDim.x >> 5; w++) {
+    all += wsum[w];
+    before += wsum[CW + w];
   }
   __syncthreads();
 }
 
+// The frontier list of the bitmap half of `stamp`, this block's slice of it.
+__device__ __forceinline__ uint32_t group_fill(const KParams &p, Ctr *c, const Group &g, uint32_t stamp, uint32_t *F,
+                                               uint32_t *wsum) {
+  const uint32_t *mh = p.mark + (stamp & 1u) * p.mwords;
+  const uint32_t per = (p.mwords + g.blocks - 1u) / g.blocks;
+  const uint32_t b = min(p.mwords, g.rank * per), e = min(p.mwords, b + per);
+  uint32_t all, before;
+  block_count_bits(mh, p.mwords, b, wsum, all, before);
+  block_fill_bits(mh, b, e, before, F, (uint32_t)p.n_nodes, c, wsum);
+  return all;
+}
+
+// Up to max_rounds rounds while the frontier has positions, but at most
+// `limit`, and nothing went wrong (arena full, device error).  A round: the
+// positions of the frontier, spread over all warps (lanes_solve, large ones by
+// the warp that met them), then, behind a barrier, the new descriptors
+// published, the bitmap half of the round after next cleared and the next
+// list written.
 template <class Cd>
-__global__ void __launch_bounds__(BLOCK, 1) k_solve_static(const KParams p, const StaticArgs a) {
-  __shared__ uint32_t smem[WARPS_PER_BLOCK * SM_WORDS];
-  __shared__ uint32_t tscr[WARPS_PER_BLOCK * TSCR * 32];
-  __shared__ unsigned long long ws[BLOCK];
-  __shared__ uint32_t s_err;
-  Ctr *c = p.ctr;
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const unsigned long long N = p.n_nodes, M = p.n_edges;
-  uint32_t *rrow = const_cast<uint32_t *>(p.rrow), *rcol = const_cast<uint32_t *>(p.rcol);
-  // -- everything that must start at zero, and the control block
-  if (tid == 0) {
-    Ctr h{};
-    h.arena = a.arena;
-    h.arena_cap = a.arena_cap;
-    h.arena_top = 1;  // word 0: the zero energy
-    h.stamp = 1;
-    *c = h;
-    a.arena[0] = 0u;
-    s_err = 0u;
-  }
-  for (unsigned long long v = tid; v < N; v += BLOCK) {
-    p.desc[v] = 0ull;
-    p.mark[v] = 0u;
-  }
-  __syncthreads();
-  // -- successor ids and update codes (k_indegree, k_check_weights); in-degrees into mark
-  uint32_t bad = 0;
-  for (unsigned long long k = tid; k < M; k += BLOCK) {
-    const uint32_t w = p.col[k];
-    if (w < N) atomicAdd(&p.mark[w], 1u);
-    else bad |= SERR_COL;
-    const uint32_t u = p.wt[k];
-    if (p.el * p.ub < 32u && (u >> (p.el * p.ub)) != 0u) bad |= SERR_WEIGHT;
-    for (uint32_t i = 0; i < p.el; i++)
-      if (((u >> (i * p.ub)) & p.um) > p.el + 1u) bad |= SERR_WEIGHT;
-  }
-  if (bad) atomicOr(&s_err, bad);
-  __syncthreads();
-  if (s_err) {
-    if (tid == 0) c->pad = s_err;
-    return;
-  }
-  // -- reverse CSR: offsets, then predecessors through a cursor kept in mark
-  block_excl_scan_n<uint32_t>(N, [&](unsigned long long v) { return (unsigned long long)p.mark[v]; }, rrow, ws);
-  for (unsigned long long v = tid; v < N; v += BLOCK) p.mark[v] = rrow[v];
-  __syncthreads();
-  for (unsigned long long v = tid; v < N; v += BLOCK)
-    for (uint32_t k = p.row[v]; k < p.row[v + 1]; k++) rcol[atomicAdd(&p.mark[p.col[k]], 1u)] = (uint32_t)v;
-  __syncthreads();
-  for (unsigned long long v = tid; v < 2ull * p.mwords; v += BLOCK) p.mark[v] = 0u;
-  __syncthreads();
-  // -- standard initialisation: {0} at the positions to reach (EnergyGame::with_reach)
-  auto is_reach = [&](unsigned long long v) { return !(p.flags[v] & 1u) && p.row[v + 1] == p.row[v]; };
-  const unsigned long long n_src = a.reach ? a.n_reach : N;
-  for (unsigned long long i = tid; i < n_src; i += BLOCK) {
-    if (a.reach) p.desc[a.reach[i]] = inl_hdr(1u);
-    else if (is_reach(i)) p.desc[i] = inl_hdr(1u);
-  }
-  __syncthreads();
-  uint32_t *sm = smem + warp * SM_WORDS;
-  for (unsigned long long b0 = (unsigned long long)warp * 32u; b0 < n_src; b0 += BLOCK) {
-    const unsigned long long i = b0 + lane;
-    bool f = false;
-    uint32_t v = 0;
-    if (i < n_src) {
-      v = a.reach ? a.reach[i] : (uint32_t)i;
-      f = a.reach ? true : is_reach(i);
-    }
-    push_preds_warp(p, c, sm, v, f, c->stamp, lane);
-  }
-  __syncthreads();
-  __shared__ uint32_t s_wsum[33];
-  {
-    const uint32_t n0 = block_fill_bits(p.mark + (c->stamp & 1u) * p.mwords, 0u, p.mwords, 0u, p.front0,
-                                        (uint32_t)N, c, s_wsum);
-    if (tid == 0) c->fsize[0] = n0;
-    __syncthreads();
-  }
-  // -- rounds (k_round + k_commit + k_fcount/k_ffill in one block)
-  uint32_t *scr = tscr + warp * (TSCR * 32) + lane;
+__device__ void group_rounds(const KParams &p, Ctr *c, const Group &g, RoundState &st, uint32_t max_rounds,
+                             uint32_t limit, uint32_t *dsm, uint32_t *wsum, uint32_t *flags) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  uint32_t *sm = dsm + warp * CWARP_WORDS;
+  uint32_t *scr = sm + W_WORDS + lane;
   const Cd cd = make_codec<Cd>(p);
-  uint32_t *arena = a.arena;
-  const unsigned long long cap = a.arena_cap;
+  uint32_t *arena = c->arena;
+  const unsigned long long cap = c->arena_cap;
   WarpAlloc wa{0, 0};
   unsigned long long w_edges = 0, w_bytes = 0, w_pos = 0;
   uint32_t t_edges = 0, t_bytes = 0, t_pos = 0;
   WarpCtx x{p, c, arena, cap, lane, sm, wa, w_edges, w_bytes, scr};
-  __shared__ uint32_t s_cur, s_fs, s_stop;
-  for (uint32_t r = 0;; r++) {
-    // one thread decides, so that every warp leaves the loop in the same round
-    if (tid == 0) {
-      s_cur = c->cur;
-      s_fs = c->fsize[s_cur];
-      s_stop = (s_fs == 0u || c->overflow || c->error) ? 1u : (r >= a.max_rounds ? 2u : 0u);
-      if (s_stop == 2u) c->pad = SERR_ROUNDS;
-    }
-    __syncthreads();
-    if (s_stop) break;
-    const uint32_t cur = s_cur, fs = s_fs;
-    const uint32_t *F = cur ? p.front1 : p.front0;
-    const uint32_t stamp = c->stamp + 1u;
-    for (uint32_t base = warp * 32u; base < fs; base += BLOCK) {
+  const uint32_t warps = g.blocks * nw, gw = warp * g.blocks + g.rank;  // neighbours on different SMs
+  for (uint32_t r = 0; r < max_rounds && st.fs != 0u && st.fs <= limit; r++) {
+    const uint32_t *F = st.cur ? p.front1 : p.front0;
+    const uint32_t stamp = st.stamp + 1u;
+    const uint32_t grab = min(32u, max(SPREAD_MIN, (st.fs + warps - 1u) / warps));
+    for (uint32_t base = gw * grab; base < st.fs; base += warps * grab) {
       const uint32_t slot = base + lane;
-      const bool active = slot < fs;
+      const bool active = lane < grab && slot < st.fs;
       const uint32_t v = active ? ld(F, slot, p.n_nodes, c) : 0u;
-      int ts = T_NONE;
       uint32_t cnt = 0, old_cnt = 0;
-      if (active)
-        ts = p.thread_path ? thread_solve(p, c, cd, arena, cap, v, scr, cnt, t_edges, t_bytes, old_cnt) : T_BIG;
+      int ts = lanes_solve(p, c, cd, arena, cap, v, active, sm, scr, lane, cnt, t_edges, t_bytes, old_cnt);
       if (ts != T_NONE && ts != T_BIG && ts != T_SKIPPED) t_pos++;
       unsigned long long nd = NONE_DESC;
       if (ts == T_CHANGED && cnt <= p.inl) {
@@ -4118,42 +4164,43 @@ __global__ void __launch_bounds__(BLOCK, 1) k_solve_static(const KParams p, cons
       }
       if (ts == T_CHANGED) t_bytes += 4u * cnt;
       if (active && ts != T_BIG && CHECK_IDX(c, slot, p.n_nodes)) p.slot_new[slot] = (ts == T_CHANGED) ? nd : NONE_DESC;
+      bool retry = ts == T_OVERFLOW, changed = ts == T_CHANGED;
       uint32_t big = __ballot_sync(FULL, ts == T_BIG);
-      bool big_changed = false;
       while (big) {
         const uint32_t l = __ffs(big) - 1u;
         big &= big - 1u;
         const uint32_t vb = __shfl_sync(FULL, v, l);
+        const bool was_empty = dcnt(ld(p.desc, vb, p.n_nodes, c)) == 0u;
         const Res rs = solve_position(x, cd, vb);
         if (rs.st != R_SKIPPED) w_pos++;
         if (lane == 0 && CHECK_IDX(c, base + l, p.n_nodes))
           p.slot_new[base + l] = (rs.st == R_CHANGED) ? rs.d : NONE_DESC;
-        if (lane == l) big_changed = rs.st == R_CHANGED;
+        if (lane == l) {
+          changed = rs.st == R_CHANGED;
+          retry = rs.st == R_OVERFLOW;
+          old_cnt = was_empty ? 0u : 1u;
+        }
       }
-      push_preds_warp(p, c, sm, v, ts == T_CHANGED || big_changed, stamp, lane);
+      push_preds_warp(p, c, sm, v, changed, stamp, lane, old_cnt == 0u);
+      if (retry) mark_push(p, v, stamp);  // again after the arena was compacted
     }
-    __syncthreads();
-    for (uint32_t i = tid; i < p.mwords; i += BLOCK) p.mark[(c->stamp & 1u) * p.mwords + i] = 0u;
-    for (uint32_t s2 = tid; s2 < fs; s2 += BLOCK) {
+    g.sync();
+    uint32_t *clear = p.mark + (st.stamp & 1u) * p.mwords;
+    for (uint32_t i = g.tid; i < p.mwords; i += g.threads) clear[i] = 0u;
+    for (uint32_t s2 = g.tid; s2 < st.fs; s2 += g.threads) {
       const unsigned long long d = p.slot_new[s2];
       if (d != NONE_DESC) {
         const uint32_t v = F[s2];
         if (CHECK_IDX(c, v, p.n_nodes)) p.desc[v] = d;
       }
     }
-    __syncthreads();
-    if (tid == 0) {
-      c->fsize[cur] = 0u;
-      c->cur = cur ^ 1u;
-      c->stamp = c->stamp + 1u;
-      c->rounds = c->rounds + 1ull;
-    }
-    __syncthreads();
-    // the next frontier, in position order, from the half this round filled
-    const uint32_t nn = block_fill_bits(p.mark + (c->stamp & 1u) * p.mwords, 0u, p.mwords, 0u,
-                                        cur ? p.front0 : p.front1, (uint32_t)N, c, s_wsum);
-    if (tid == 0) c->fsize[cur ^ 1u] = nn;
-    __syncthreads();
+    if (threadIdx.x == 0) *flags = *(volatile uint32_t *)&c->overflow | *(volatile uint32_t *)&c->error;
+    st.fs = group_fill(p, c, g, stamp, st.cur ? p.front0 : p.front1, wsum);  // its barriers cover *flags
+    st.cur ^= 1u;
+    st.stamp = stamp;
+    st.rounds++;
+    g.sync();
+    if (*flags) break;
   }
   unsigned long long te = t_edges, tb = t_bytes, tp = t_pos;
 #pragma unroll
@@ -4162,33 +4209,242 @@ __global__ void __launch_bounds__(BLOCK, 1) k_solve_static(const KParams p, cons
     tb += __shfl_xor_sync(FULL, tb, o);
     tp += __shfl_xor_sync(FULL, tp, o);
   }
-  if (lane == 0) {
+  if (lane == 0 && (tp | w_pos)) {
     atomicAdd(&c->positions, tp + w_pos);
     atomicAdd(&c->edges, te + w_edges);
     atomicAdd(&c->bytes, tb + w_bytes);
   }
+}
+
+// Rounds of an upload by one cluster: the state is taken from the control
+// block and left there as k_commit / k_ffill leave it.
+template <class Cd>
+__global__ void __launch_bounds__(CT, 1) k_rounds_cluster(const KParams p, uint32_t max_rounds, uint32_t limit) {
+  extern __shared__ uint32_t dsm[];
+  __shared__ uint32_t wsum[2 * CW + 2], s_flags;
+  Ctr *c = p.ctr;
+  const Group g = this_group();
+  RoundState st{c->cur, c->fsize[c->cur], c->stamp, 0u};
+  if (c->halt) st.fs = 0u;
+  const bool idle = st.fs == 0u || st.fs > limit;
+  g.sync();  // every block has read the state
+  if (idle) return;
+  group_rounds<Cd>(p, c, g, st, max_rounds, limit, dsm, wsum, &s_flags);
+  if (g.tid == 0) {
+    c->fsize[0] = st.cur ? 0u : st.fs;
+    c->fsize[1] = st.cur ? st.fs : 0u;
+    c->cur = st.cur;
+    c->stamp = st.stamp;
+    c->rounds = c->rounds + st.rounds;
+    c->next_slot = 0u;
+    c->nbig = 0u;
+    c->next_big = 0u;
+    if (c->overflow) c->halt = 1u;
+  }
+}
+
+// out[v] = sum of cnt(u) for u < v, out[n] = the total; one block.  ws: 34
+// words of shared memory.
+template <class T, class F>
+__device__ void block_excl_scan_n(unsigned long long n, F cnt, T *out, unsigned long long *ws) {
+  constexpr uint32_t ITEMS = 8;
+  unsigned long long carry = 0;
+  for (unsigned long long t0 = 0; t0 < n; t0 += (unsigned long long)blockDim.x * ITEMS) {
+    const unsigned long long b = t0 + (unsigned long long)threadIdx.x * ITEMS;
+    uint32_t x[ITEMS];
+    unsigned long long sum = 0, total;
+#pragma unroll
+    for (uint32_t i = 0; i < ITEMS; i++) {
+      x[i] = b + i < n ? cnt(b + i) : 0u;
+      sum += x[i];
+    }
+    unsigned long long acc = carry + block_excl_scan(sum, ws, total);
+#pragma unroll
+    for (uint32_t i = 0; i < ITEMS; i++)
+      if (b + i < n) {
+        out[b + i] = (T)acc;
+        acc += x[i];
+      }
+    carry += total;
+  }
+  if (threadIdx.x == 0) out[n] = (T)carry;
   __syncthreads();
-  if (c->overflow) {
-    if (tid == 0) c->pad |= SERR_ARENA;
+}
+
+// One game from its host arrays to its result lists in one launch of a
+// cluster of blocks, or of one block (geq_energy_game_run_static).
+template <class Cd>
+__global__ void __launch_bounds__(CT, 1) k_solve_static(const KParams p, const StaticArgs a) {
+  extern __shared__ uint32_t dsm[];
+  __shared__ uint32_t wsum[2 * CW + 2], s_flags;
+  __shared__ unsigned long long ws[34];
+  Ctr *c = p.ctr;
+  const Group g = this_group();
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const unsigned long long N = p.n_nodes, M = p.n_edges;
+  uint32_t *rrow = const_cast<uint32_t *>(p.rrow), *rcol = const_cast<uint32_t *>(p.rcol);
+  for (unsigned long long i = g.tid; i < a.in_vecs; i += g.threads) a.dst[i] = a.h_in[i];
+  // -- everything that must start at zero, and the control block
+  if (g.tid == 0) {
+    Ctr h{};
+    h.arena = a.arena;
+    h.arena_cap = a.arena_cap;
+    h.arena_top = 1;  // word 0: the zero energy
+    h.stamp = 1;
+    *c = h;
+    a.arena[0] = 0u;
+  }
+  for (unsigned long long v = g.tid; v < N; v += g.threads) {
+    p.desc[v] = 0ull;
+    p.mark[v] = 0u;
+  }
+  g.sync();
+  // -- successor ids and update codes (k_indegree, k_check_weights); in-degrees into mark
+  uint32_t bad = 0;
+  for (unsigned long long k = g.tid; k < M; k += g.threads) {
+    const uint32_t w = p.col[k];
+    if (w < N) atomicAdd(&p.mark[w], 1u);
+    else bad |= SERR_COL;
+    const uint32_t u = p.wt[k];
+    if (p.el * p.ub < 32u && (u >> (p.el * p.ub)) != 0u) bad |= SERR_WEIGHT;
+    for (uint32_t i = 0; i < p.el; i++)
+      if (((u >> (i * p.ub)) & p.um) > p.el + 1u) bad |= SERR_WEIGHT;
+  }
+  if (bad) atomicOr(&c->pad, bad);
+  g.sync();
+  if (c->pad) {
+    if (a.h_ctr && g.tid == 0) *a.h_ctr = *c;
     return;
   }
-  if (c->pad || c->error) return;
+  // -- reverse CSR: offsets, then predecessors through a cursor kept in mark
+  if (g.rank == 0) {
+    block_excl_scan_n<uint32_t>(N, [&](unsigned long long v) { return p.mark[v]; }, rrow, ws);
+    for (unsigned long long v = threadIdx.x; v < N; v += blockDim.x) p.mark[v] = rrow[v];
+  }
+  g.sync();
+  for (unsigned long long v = g.tid; v < N; v += g.threads)
+    for (uint32_t k = p.row[v]; k < p.row[v + 1]; k++) rcol[atomicAdd(&p.mark[p.col[k]], 1u)] = (uint32_t)v;
+  g.sync();
+  for (unsigned long long v = g.tid; v < 2ull * p.mwords; v += g.threads) p.mark[v] = 0u;
+  // -- standard initialisation: {0} at the positions to reach (EnergyGame::with_reach)
+  auto is_reach = [&](unsigned long long v) { return !(p.flags[v] & 1u) && p.row[v + 1] == p.row[v]; };
+  const unsigned long long n_src = a.reach ? a.n_reach : N;
+  for (unsigned long long i = g.tid; i < n_src; i += g.threads) {
+    if (a.reach) p.desc[a.reach[i]] = inl_hdr(1u);
+    else if (is_reach(i)) p.desc[i] = inl_hdr(1u);
+  }
+  g.sync();
+  uint32_t *sm = dsm + warp * CWARP_WORDS;
+  for (unsigned long long b0 = (unsigned long long)(g.tid >> 5) * 32u; b0 < n_src; b0 += g.threads) {
+    const unsigned long long i = b0 + lane;
+    bool f = false;
+    uint32_t v = 0;
+    if (i < n_src) {
+      v = a.reach ? a.reach[i] : (uint32_t)i;
+      f = a.reach ? true : is_reach(i);
+    }
+    push_preds_warp(p, c, sm, v, f, 1u, lane);
+  }
+  g.sync();
+  RoundState st{0u, 0u, 1u, 0u};
+  st.fs = group_fill(p, c, g, st.stamp, p.front0, wsum);
+  g.sync();
+  group_rounds<Cd>(p, c, g, st, a.max_rounds, ~0u, dsm, wsum, &s_flags);
+  g.sync();
+  if (g.tid == 0) {
+    c->rounds = st.rounds;
+    c->pad = c->overflow ? SERR_ARENA : (!c->error && st.fs) ? SERR_ROUNDS : 0u;
+  }
+  g.sync();
+  if (c->pad || c->error) {
+    if (a.h_ctr && g.tid == 0) *a.h_ctr = *c;
+    return;
+  }
   // -- result lists (k_desc_counts + scan + k_gather) behind the arena's used part
-  block_excl_scan_n<unsigned long long>(N, [&](unsigned long long v) { return (unsigned long long)dcnt(p.desc[v]); },
-                                        a.out_off, ws);
+  if (g.rank == 0)
+    block_excl_scan_n<unsigned long long>(N, [&](unsigned long long v) { return dcnt(p.desc[v]); }, a.out_off, ws);
+  g.sync();
   const unsigned long long top = c->arena_top, total = a.out_off[N];
-  if (top + total > cap) {
-    if (tid == 0) c->pad = SERR_ARENA;
-    return;
+  const bool to_host = a.h_data && total <= a.h_cap;
+  const bool full = !to_host && top + total > a.arena_cap;
+  if (g.tid == 0) {
+    if (full) c->pad = SERR_ARENA;
+    if (a.h_ctr) *a.h_ctr = *c;
   }
-  uint32_t *out = arena + top;
-  for (unsigned long long v = warp; v < N; v += WARPS_PER_BLOCK) {
+  if (full) return;
+  if (a.h_off)
+    for (unsigned long long v = g.tid; v <= N; v += g.threads) a.h_off[v] = a.out_off[v];
+  uint32_t *out = to_host ? a.h_data : a.arena + top;
+  for (unsigned long long v = g.tid; v < N; v += g.threads) {
     const unsigned long long d = p.desc[v];
     const uint32_t n = dcnt(d);
     const unsigned long long go = a.out_off[v];
-    for (uint32_t q = lane; q < n; q += 32u)
-      out[go + q] = dinl(d) ? ((uint32_t)(d >> (q * p.ib)) & p.ibm) : arena[doff(d) + q];
+    for (uint32_t q = 0; q < n; q++)
+      out[go + q] = dinl(d) ? ((uint32_t)(d >> (q * p.ib)) & p.ibm) : a.arena[doff(d) + q];
   }
+}
+
+// One launch of a cluster of `blocks` blocks.
+template <class... P, class... A>
+static cudaError_t launch_cluster(void (*f)(P...), uint32_t blocks, uint32_t warps, cudaStream_t S, const A &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(32 * warps);
+  cfg.dynamicSmemBytes = cluster_smem(warps);
+  cfg.stream = S;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = blocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = blocks > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, f, args...);
+}
+// Shared memory and cluster size of the cluster kernels on the current device.
+template <class F>
+static cudaError_t cluster_attrs(F *f) {
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem(CW));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e;
+}
+static geq_status cluster_setup(uint32_t &blocks) {
+  CU(cluster_attrs(k_rounds_cluster<CodecStd>));
+  CU(cluster_attrs(k_rounds_cluster<CodecGen>));
+  CU(cluster_attrs(k_solve_static<CodecStd>));
+  CU(cluster_attrs(k_solve_static<CodecGen>));
+  for (blocks = 16; blocks > 1; blocks /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(CT);
+    cfg.dynamicSmemBytes = cluster_smem(CW);
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0, m = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_rounds_cluster<CodecStd>, &cfg) == cudaSuccess && n > 0 &&
+        cudaOccupancyMaxActiveClusters(&m, k_solve_static<CodecStd>, &cfg) == cudaSuccess && m > 0)
+      break;
+    cudaGetLastError();
+  }
+  return GEQ_OK;
+}
+static geq_status launch_rounds_cluster(const Engine &E, const KParams &kp, bool generic, uint32_t max_rounds,
+                                        uint32_t limit) {
+  const Engine::State &s = *E.st;
+  CU(generic ? launch_cluster(k_rounds_cluster<CodecGen>, s.cluster, CW, s.stream, kp, max_rounds, limit)
+             : launch_cluster(k_rounds_cluster<CodecStd>, s.cluster, CW, s.stream, kp, max_rounds, limit));
+  return GEQ_OK;
+}
+static geq_status launch_solve_static(const KParams &kp, const StaticArgs &sa, bool generic, uint32_t blocks,
+                                      cudaStream_t S) {
+  if (kp.n_nodes <= STATIC_ONE_BLOCK) blocks = 1;
+  const uint32_t warps = blocks == 1 && kp.n_nodes <= STATIC_FEW_WARPS ? 8u : CW;
+  CU(generic ? launch_cluster(k_solve_static<CodecGen>, blocks, warps, S, kp, sa)
+             : launch_cluster(k_solve_static<CodecStd>, blocks, warps, S, kp, sa));
+  return GEQ_OK;
 }
 
 // Device address of the scratch on the current device.  Looked up on every
@@ -4313,9 +4569,7 @@ geq_status Engine::run_static(int device, const geq_game_graph &g, const uint32_
   if (N) CU(cudaMemcpyAsync(base + L.flags, g.attacker_pos, N, cudaMemcpyHostToDevice, S));
   if (to_reach && n_reach) CU(cudaMemcpyAsync(base + L.reach, to_reach, (size_t)n_reach * 4, cudaMemcpyHostToDevice, S));
   const bool generic = !conf.standard() || (tuning.flags & GEQ_TUNE_FORCE_GENERIC);
-  if (generic) k_solve_static<CodecGen><<<1, BLOCK, 0, S>>>(kp, sa);
-  else k_solve_static<CodecStd><<<1, BLOCK, 0, S>>>(kp, sa);
-  CU(cudaGetLastError());
+  if ((rc = launch_solve_static(kp, sa, generic, 1, S))) return rc;
   Ctr h{};
   CU(cudaMemcpyAsync(&h, kp.ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, S));
   CU(cudaMemcpyAsync(offsets, sa.out_off, (N + 1) * 8, cudaMemcpyDeviceToHost, S));
@@ -4351,9 +4605,9 @@ geq_status Engine::run_static(int device, const geq_game_graph &g, const uint32_
 }
 
 
-// One small game in one launch of the one-block solver, in a pooled device
-// block: one upload from page-locked staging, one kernel, two read-backs.  A
-// game whose lists outgrow the block's arena is left to the general path
+// One small game in one launch, in a pooled device block: the kernel reads the
+// game from page-locked staging and writes the lists to page-locked memory, so
+// the call waits once.  A game whose lists outgrow the block's arena is left to the general path
 // (handled = false), as is everything outside the limits.
 geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &handled) {
   handled = false;
@@ -4387,18 +4641,26 @@ geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &han
   StaticArgs sa;
   block_params(L, base, bytes, N, M, conf, tuning, true, gi.n_reach, kp, sa);
   CU(cudaEventRecord(s.ev0, S));
-  CU(cudaMemcpyAsync(base, H, L.rrow, cudaMemcpyHostToDevice, S));
-  if (!conf.standard()) k_solve_static<CodecGen><<<1, BLOCK, 0, S>>>(kp, sa);
-  else k_solve_static<CodecStd><<<1, BLOCK, 0, S>>>(kp, sa);
-  CU(cudaGetLastError());
   sol.n_offsets = N + 1;
+  const unsigned long long room = 4 * N + 256;  // energies the kernel writes to the host by itself
   if (!sol.off_buf.alloc(s.hpool, (N + 1) * 8)) return fail(GEQ_ERR_OUT_OF_MEMORY, "host memory for offsets");
-  CU(cudaMemcpyAsync(s.h_ctr, kp.ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, S));
-  CU(cudaMemcpyAsync(sol.off_buf.p, sa.out_off, (N + 1) * 8, cudaMemcpyDeviceToHost, S));
+  if (!sol.data_buf.alloc(s.hpool, room * 4)) return fail(GEQ_ERR_OUT_OF_MEMORY, "host memory for %llu words", room);
+  sa.h_in = (const uint4 *)H;
+  sa.dst = (uint4 *)base;
+  sa.in_vecs = L.rrow / sizeof(uint4);
+  sa.h_ctr = s.h_ctr;
+  // (a block from the heap, when no page-locked one could be had, is not the device's to write)
+  sa.h_off = sol.off_buf.pool ? (unsigned long long *)sol.off_buf.p : nullptr;
+  sa.h_data = sol.data_buf.pool && sa.h_off ? (uint32_t *)sol.data_buf.p : nullptr;
+  sa.h_cap = sa.h_data ? room : 0;
+  if ((rc = launch_solve_static(kp, sa, !conf.standard(), s.cluster, S))) return rc;
+  if (!sa.h_off) CU(cudaMemcpyAsync(sol.off_buf.p, sa.out_off, (N + 1) * 8, cudaMemcpyDeviceToHost, S));
+  CU(cudaEventRecord(s.ev1, S));
   CU(cudaStreamSynchronize(S));
   const Ctr h = *s.h_ctr;
   if ((h.pad & SERR_ARENA) || (h.error & ~DERR_BOUNDS)) {
     sol.off_buf.reset();
+    sol.data_buf.reset();
     return GEQ_OK;  // the general path grows its arena
   }
   handled = true;
@@ -4408,10 +4670,13 @@ geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &han
   if (h.pad & SERR_ROUNDS) return fail(GEQ_ERR_TIMEOUT, "no fixpoint after %u rounds", sa.max_rounds);
   const unsigned long long total = ((const uint64_t *)sol.off_buf.p)[N];
   sol.n_words = total;
-  if (!sol.data_buf.alloc(s.hpool, total * 4)) return fail(GEQ_ERR_OUT_OF_MEMORY, "host memory for %llu words", total);
-  if (total) CU(cudaMemcpyAsync(sol.data_buf.p, sa.arena + h.arena_top, total * 4, cudaMemcpyDeviceToHost, S));
-  CU(cudaEventRecord(s.ev1, S));
-  CU(cudaStreamSynchronize(S));
+  if (total > sa.h_cap) {
+    if (total > room && !sol.data_buf.alloc(s.hpool, total * 4))
+      return fail(GEQ_ERR_OUT_OF_MEMORY, "host memory for %llu words", total);
+    CU(cudaMemcpyAsync(sol.data_buf.p, sa.arena + h.arena_top, total * 4, cudaMemcpyDeviceToHost, S));
+    CU(cudaEventRecord(s.ev1, S));
+    CU(cudaStreamSynchronize(S));
+  }
   float ms = 0.f;
   cudaEventElapsedTime(&ms, s.ev0, s.ev1);
   sol.energy_size = 1;

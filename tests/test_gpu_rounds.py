@@ -94,6 +94,30 @@ def solve(geq, ctx, game):
     return o, d
 
 
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 255, 256, 257, 400, 401, 4096, 4097, 32768, 32769])
+@pytest.mark.parametrize("form", ["run", "batch", "static"])
+def test_launch_forms(geq, ctx, n, form):
+    """Sizes at the lines between one block, a cluster and graphs of rounds,
+    through the calls that take them: one game (a launch of its own up to
+    32,768 positions), the same game beside an empty one (an upload and rounds),
+    and the allocation-free call."""
+    row, col, wt, att, _, _, _ = make_game(100 + n, max(n, 2), 2.5, 1)
+    if n == 1:
+        row, col, wt, att = row[:2] * 0, col[:0], wt[:0], att[1:]
+    g = geq.GameGraph.from_csr(row, col, wt, att, geq.EnergyConf.STANDARD)
+    if form == "static":
+        o, d, _ = geq.run_static(g, ctx)
+    elif form == "run":
+        offs, data, _ = geq.run_batch_raw([g], ctx)
+        o, d = offs[0], data[0]
+    else:
+        offs, data, _ = geq.run_batch_raw([g, geq.GameGraph.empty(geq.EnergyConf.STANDARD)], ctx)
+        o, d = offs[0], data[0]
+    exp = ora.run_game(6, 3, row, col, wt, att, ora.standard_reach(row, att)).lists()
+    for v in range(len(att)):
+        assert canon(d[int(o[v]):int(o[v + 1])]) == canon(exp[v]), f"position {v}"
+
+
 @pytest.mark.parametrize("seed,n,mean_deg,merges", [(1, 6000, 3.0, 1), (2, 9000, 1.6, 2), (3, 5000, 7.0, 3),
                                                     (4, 7000, 2.5, 0)])
 def test_small_and_large_rounds_agree(geq, ctx, seed, n, mean_deg, merges):
