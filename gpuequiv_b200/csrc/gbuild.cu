@@ -8,6 +8,7 @@
 // loop's queries and geq_equivalences); and
 // TransitionSystem::signature_refinement of many systems at once
 // (geq_lts_signature_refinement_batch).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <chrono>
@@ -438,10 +439,13 @@ __device__ void gen_attack_warp(const View &v, uint32_t i, uint32_t *bm, uint32_
 }
 
 // End of one level inside the graph's WHILE node: run the next level while
-// the loop may go on, at most ctr[1] levels per graph launch (ctr[0] counts).
+// the loop may go on, at most ctr[1] levels per graph launch (ctr[0] counts),
+// and until the frontier has shrunk to what one cluster expands faster
+// (ctr[2], reached from above).
 __global__ void k_level_cond(cudaGraphConditionalHandle h, const unsigned long long *go, uint32_t *ctr) {
   const uint32_t k = ++ctr[0];
-  cudaGraphSetConditional(h, (*go != 0ull && k < ctr[1]) ? 1u : 0u);
+  const unsigned long long *t = go - T_GO;
+  cudaGraphSetConditional(h, (*go != 0ull && k < ctr[1] && t[T_F] > ctr[2]) ? 1u : 0u);
 }
 
 __global__ void __launch_bounds__(GH_WARPS * 32) k_gen_heavy(View v, const unsigned long long *go) {
@@ -451,6 +455,276 @@ __global__ void __launch_bounds__(GH_WARPS * 32) k_gen_heavy(View v, const unsig
   const uint32_t nh = v.ctl->n_heavy;
   for (uint32_t h = blockIdx.x * GH_WARPS + wib; h < nh; h += gridDim.x * GH_WARPS)
     gen_attack_warp(v, v.hq[h], bm_all[wib], lane);
+}
+
+// ---- levels with small frontiers, inside one launch ---------------------------
+// A level as launches of its own is ~20 kernels, each of which costs its launch
+// and drain (about 3 us) however few positions there are; a system of a few
+// hundred states has 5 to 30 such levels.  A cluster of blocks runs the same
+// functors phase after phase with the cluster's hardware barrier between them
+// (nothing spins), level after level, until the frontier runs empty, outgrows
+// `limit` or a buffer must grow.
+namespace cg = cooperative_groups;
+constexpr uint32_t CLW = 16;  // warps per block
+constexpr uint32_t CLT = 32 * CLW;
+constexpr size_t CL_SMEM = (size_t)CLW * GH_BM_WORDS * 4;
+
+struct Cluster {
+  uint32_t rank, blocks, tid, threads, warp, warps;
+  __device__ __forceinline__ void sync() const { cg::this_cluster().sync(); }
+  // f(i) for i < n; neighbouring warps of items sit on different SMs
+  template <class F>
+  __device__ __forceinline__ void each(uint32_t n, const F &f) const {
+    for (uint32_t i = tid; i < n; i += threads) f(i);
+  }
+};
+__device__ __forceinline__ Cluster this_cluster_threads() {
+  const cg::cluster_group cl = cg::this_cluster();
+  Cluster g;
+  g.rank = cl.block_rank();
+  g.blocks = cl.num_blocks();
+  g.warp = (threadIdx.x >> 5) * g.blocks + g.rank;
+  g.warps = g.blocks * (blockDim.x >> 5);
+  g.tid = g.warp * 32u + (threadIdx.x & 31u);
+  g.threads = g.warps * 32u;
+  return g;
+}
+
+struct ScanSh {
+  unsigned long long sum[3], pre[3], tot[3];
+  unsigned long long ws[CLW + 1];
+};
+// exclusive scan over the block's threads, one value each; total to all
+__device__ __forceinline__ unsigned long long cl_block_scan(unsigned long long x, unsigned long long *ws,
+                                                            unsigned long long &total) {
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  unsigned long long inc = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long y = __shfl_up_sync(FULLMASK, inc, o);
+    if (lane >= (uint32_t)o) inc += y;
+  }
+  if (lane == 31u) ws[w] = inc;
+  __syncthreads();
+  unsigned long long before = 0, all = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < CLW; k++) {
+    const unsigned long long y = ws[k];
+    if (k < w) before += y;
+    all += y;
+  }
+  __syncthreads();
+  total = all;
+  return before + inc - x;
+}
+// Exclusive scans of up to three arrays in(r, i), i < n[r], to out[r]; totals to
+// sh.tot (in every block).  Block b scans the b-th slice; the blocks exchange
+// their sums through distributed shared memory.  Inputs must be visible to
+// the block that scans them (a barrier before), outputs are after the next one.
+template <int R, class In>
+__device__ __forceinline__ void cl_scan(const Cluster &g, const uint32_t (&n)[R], const In &in,
+                                        uint32_t *const (&out)[R], ScanSh &sh) {
+  const cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const uint32_t per = (n[r] + g.blocks - 1u) / g.blocks, b = min(n[r], g.rank * per), e = min(n[r], b + per);
+    unsigned long long s = 0, total;
+    for (uint32_t i = b + threadIdx.x; i < e; i += CLT) s += in(r, i);
+    cl_block_scan(s, sh.ws, total);
+    if (threadIdx.x == 0) sh.sum[r] = total;
+  }
+  cl.sync();
+  if (threadIdx.x < 32u) {
+    const uint32_t lane = threadIdx.x;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const unsigned long long x = lane < g.blocks ? *cl.map_shared_rank(&sh.sum[r], lane) : 0ull;
+      unsigned long long all = x, pre = lane < g.rank ? x : 0ull;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        all += __shfl_xor_sync(FULLMASK, all, o);
+        pre += __shfl_xor_sync(FULLMASK, pre, o);
+      }
+      if (lane == 0) {
+        sh.pre[r] = pre;
+        sh.tot[r] = all;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const uint32_t per = (n[r] + g.blocks - 1u) / g.blocks, b = min(n[r], g.rank * per), e = min(n[r], b + per);
+    unsigned long long carry = sh.pre[r];
+    for (uint32_t t0 = b; t0 < e; t0 += CLT) {
+      const uint32_t i = t0 + threadIdx.x;
+      const uint32_t x = i < e ? in(r, i) : 0u;
+      unsigned long long total;
+      const unsigned long long ex = cl_block_scan(x, sh.ws, total);
+      if (i < e) out[r][i] = (uint32_t)(carry + ex);
+      carry += total;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(CLT, 1) k_levels_cluster(View v, uint32_t start, uint32_t n_starts, uint32_t limit) {
+  extern __shared__ uint32_t bm_all[];
+  __shared__ ScanSh sh;
+  const Cluster g = this_cluster_threads();
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t *bm = bm_all + (threadIdx.x >> 5) * GH_BM_WORDS;
+  const bool one = g.rank == 0 && threadIdx.x == 0;
+  // the new positions' job-local ids, then the counts of the level
+  auto locals = [&](uint32_t cnt) {
+    g.each(cnt, LocalBF{v});
+    g.sync();
+    g.each(cnt, LocalCF{v});
+    g.sync();
+  };
+  if (start) {
+    // the empty set is set 0; level 0: Attack(p0[t], {q0[t]}), numbered in order
+    if (one) {
+      v.sstart[0] = 0u;
+      v.slen[0] = 0u;
+      *v.ctl = Ctl{0u, 1u, 0u, 0u};
+      SetRehashF{v}(0u);
+    }
+    g.each(n_starts, StartF{v});
+    g.sync();
+    g.each(n_starts, SetProbeF{v});
+    g.sync();
+    g.each(n_starts, SetNewF{v});
+    g.sync();
+    g.each(n_starts, SetFillF{v});
+    g.each(n_starts, SuccProbeF{v, true});
+    g.sync();
+    const uint32_t n[1] = {n_starts};
+    uint32_t *const out[1] = {v.srank};
+    g.each(n_starts, SuccFlagF{v});
+    g.sync();
+    cl_scan<1>(g, n, [&](int, uint32_t i) { return v.snew[i]; }, out, sh);
+    const uint32_t cnt = (uint32_t)sh.tot[0];
+    if (one) v.t[T_NEW] = cnt;
+    g.sync();
+    g.each(n_starts, SuccNewF{v});
+    g.sync();
+    g.each(n_starts, SuccFillF{v});
+    g.each(cnt, LocalAF{v});
+    g.sync();
+    locals(cnt);
+    if (one) {
+      v.t[T_NN] = cnt;
+      v.t[T_F] = cnt;
+      v.t[T_GO] = 1ull;
+    }
+  }
+  if (one) v.ctl->n_heavy = 0u;
+  g.sync();
+  for (;;) {
+    const unsigned long long F = v.t[T_F];
+    if (!v.t[T_GO] || F > limit) break;
+    if (F == 0 || F > v.capF) {
+      g.sync();  // every thread has read the state
+      if (one) {
+        v.t[T_GO] = 0ull;
+        v.t[F == 0 ? T_DONE : T_STALL] = 1ull;
+      }
+      break;
+    }
+    const uint32_t f = (uint32_t)F;
+    g.each(f, CountF{v});
+    g.sync();
+    {
+      const uint32_t n[3] = {f, f, f};
+      uint32_t *const out[3] = {v.off_s, v.off_e, v.off_c};
+      cl_scan<3>(g, n, [&](int r, uint32_t i) { return r == 0 ? v.ub_s[i] : r == 1 ? v.ub_e[i] : v.ub_c[i]; }, out, sh);
+    }
+    const unsigned long long S = sh.tot[0], E = sh.tot[1], C = sh.tot[2];
+    const bool fits = level_fits(v, S, E, C);
+    if (one) {
+      v.t[T_S] = S;
+      v.t[T_E] = E;
+      v.t[T_C] = C;
+    }
+    g.sync();
+    if (!fits) {
+      if (one) {
+        v.t[T_GO] = 0ull;
+        v.t[T_STALL] = 1ull;
+      }
+      break;
+    }
+    const uint32_t ns = (uint32_t)S, nc = (uint32_t)C;
+    // light positions from the first warps on, the others from the last
+    g.each(f, GenF{v});
+    if (v.heavy_min != 0xffffffffu) {
+      const uint32_t nh = v.ctl->n_heavy;
+      for (uint32_t h = g.warps - 1u - g.warp; h < nh; h += g.warps) gen_attack_warp(v, v.hq[h], bm, lane);
+    }
+    g.sync();
+    g.each(nc, SetProbeF{v});
+    g.sync();
+    g.each(nc, SetNewF{v});
+    g.sync();
+    g.each(nc, SetFillF{v});
+    g.each(ns, SuccProbeF{v, true});
+    g.sync();
+    g.each(ns, SuccFlagF{v});
+    g.sync();
+    {
+      const uint32_t n[2] = {ns, f};
+      uint32_t *const out[2] = {v.srank, v.feoff};
+      cl_scan<2>(g, n, [&](int r, uint32_t i) { return r == 0 ? v.snew[i] : v.fcnt[i]; }, out, sh);
+    }
+    const uint32_t cnt = (uint32_t)sh.tot[0];
+    if (one) {
+      v.t[T_NEW] = cnt;
+      v.t[T_EDGE] = sh.tot[1];
+    }
+    g.sync();
+    g.each(ns, SuccNewF{v});
+    g.sync();
+    g.each(ns, SuccFillF{v});
+    g.each(cnt, LocalAF{v});
+    g.sync();
+    g.each(f, EdgeF{v});
+    locals(cnt);
+    if (one) {
+      level_end(v);
+      v.ctl->n_heavy = 0u;
+    }
+    g.sync();
+  }
+  cg::this_cluster().sync();  // distributed shared memory is read no more
+}
+
+// The per-job CSR of a small batch (PermF ... RowEndF) in one launch.
+__global__ void __launch_bounds__(CLT, 1) k_assemble_cluster(View v, Out o, uint32_t N) {
+  __shared__ ScanSh sh;
+  const Cluster g = this_cluster_threads();
+  const uint32_t J = v.n_jobs;
+  {
+    const uint32_t n[1] = {J};
+    uint32_t *const out[1] = {o.jbase};
+    cl_scan<1>(g, n, [&](int, uint32_t i) { return v.jcount[i]; }, out, sh);
+  }
+  const unsigned long long tn = sh.tot[0];
+  g.sync();
+  g.each(N, PermF{v, o});
+  g.sync();
+  {
+    const uint32_t n[1] = {N};
+    uint32_t *const out[1] = {o.frow};
+    cl_scan<1>(g, n, [&](int, uint32_t i) { return o.frl[i]; }, out, sh);
+  }
+  if (g.rank == 0 && threadIdx.x == 0) {
+    v.t[T_N] = tn;
+    v.t[T_EDGE] = sh.tot[0];
+  }
+  g.sync();
+  g.each(N, RowsF{v, o});
+  g.each(J, RowEndF{v, o});
+  cg::this_cluster().sync();
 }
 
 // Backend of the level loop: stream-ordered allocation, kernels and copies on
@@ -587,13 +861,13 @@ struct DevBackend {
   cudaGraphExec_t gexec = nullptr;
   cudaGraphConditionalHandle cond = 0;
   uint32_t *d_loop = nullptr;  // [levels run in this launch, limit]
-  uint32_t h_loop[2] = {0, 0};
+  uint32_t h_loop[3] = {0, 0, 0};
   uint32_t graph_launches = 0, mark = 0;
   bool plain = false;  // levels as plain launches, one per host sync (profilers see every kernel)
   bool has_graph() const { return gexec != nullptr; }
   void begin_capture() {
     if (plain) return;  // the level that "capture" enqueues runs as it is
-    if (!d_loop) d_loop = (uint32_t *)alloc(2 * sizeof(uint32_t));
+    if (!d_loop) d_loop = (uint32_t *)alloc(sizeof(h_loop));
     if (!d_loop) note(cudaErrorMemoryAllocation);
     mark = launches;
     note(cudaGraphCreate(&graph, 0));
@@ -621,8 +895,70 @@ struct DevBackend {
     if (!gexec) return;
     h_loop[0] = 0;
     h_loop[1] = limit;
+    h_loop[2] = cluster_blocks ? CL_FRONTIER / 2 : 0u;
     note(cudaMemcpyAsync(d_loop, h_loop, sizeof(h_loop), cudaMemcpyHostToDevice, s));
     note(cudaGraphLaunch(gexec, s));
+  }
+  // ---- small frontiers in one launch of a cluster ----
+  static constexpr bool kCluster = true;
+  // Levels of at most this many positions are expanded by one cluster.  On one
+  // B200, median per call with the line at none / 1,024 / 4,096 / 16,384:
+  // twelve compare() calls on systems with games of up to 20,000 positions
+  // 26.2 / 14.5 / 14.3 / 14.3 ms, equivalences() of a 40-state system (25,000
+  // positions) 4.7 / 4.3 / 2.8 / 3.3 ms, 512 queries together 28.3 / 22.9 /
+  // 22.9 / 22.9 ms, equivalences() of a 3,000-state system 54.6 / 45.0 / 45.4 /
+  // 46.5 ms.  (A launch of levels as a graph stops at half of it.)
+  static constexpr uint32_t CL_FRONTIER = 4096;
+  uint32_t cluster_blocks = 0;  // 0: none
+  bool cluster_ok(uint32_t items) const { return cluster_blocks && !plain && items <= CL_FRONTIER; }
+  template <class... P, class... A>
+  void launch_cluster(void (*f)(P...), size_t smem, const A &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster_blocks);
+    cfg.blockDim = dim3(CLT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = cluster_blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    note(cudaLaunchKernelEx(&cfg, f, args...));
+    launches++;
+  }
+  void cluster_levels(const View &v, bool start, uint32_t n_starts) {
+    launch_cluster(k_levels_cluster, CL_SMEM, v, start ? 1u : 0u, n_starts, CL_FRONTIER);
+  }
+  void cluster_assemble(const View &v, const Out &o, uint32_t N) { launch_cluster(k_assemble_cluster, 0, v, o, N); }
+  // Sets the kernels up on the current device; the blocks of a cluster, 0 when
+  // even 8 do not fit.
+  static uint32_t cluster_setup() {
+    auto attrs = [](auto *f, size_t smem) {
+      cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      return e;
+    };
+    if (attrs(k_levels_cluster, CL_SMEM) != cudaSuccess || attrs(k_assemble_cluster, 0) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    for (uint32_t b = 16; b >= 8; b /= 2) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(b);
+      cfg.blockDim = dim3(CLT);
+      cfg.dynamicSmemBytes = CL_SMEM;
+      cudaLaunchAttribute at = {};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = b;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, k_levels_cluster, &cfg) == cudaSuccess && n > 0) return b;
+      cudaGetLastError();
+    }
+    return 0;
   }
   // kernel launches of the levels that ran
   void note_levels(unsigned long long levels) { launches += (uint32_t)(levels * graph_launches); }
@@ -704,8 +1040,10 @@ static geq_status device_build(Engine &eng, int device, uint32_t n_jobs, const L
   // freed blocks cached in this process instead of returning them at every
   // synchronisation
   static std::once_flag pool_once[64];
+  static uint32_t cluster_blocks[64] = {};
   if (device >= 0 && device < 64)
     std::call_once(pool_once[device], [device]() {
+      cluster_blocks[device] = gb::DevBackend::cluster_setup();
       cudaMemPool_t pool;
       if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
         uint64_t keep = ~0ull;
@@ -719,6 +1057,7 @@ static geq_status device_build(Engine &eng, int device, uint32_t n_jobs, const L
   // GEQ_TUNE_NO_GRAPH: levels as plain launches (ncu does not profile the
   // kernels of a graph with conditional nodes)
   be.plain = (eng.tuning.flags & GEQ_TUNE_NO_GRAPH) != 0;
+  be.cluster_blocks = device >= 0 && device < 64 ? cluster_blocks[device] : 0u;
   // stage the LTSs: soff | slab | stgt | sjob | p0 | q0
   const auto t0 = clk::now();
   const size_t o_soff = 0, o_slab = o_soff + (NS + 1) * 4, o_stgt = o_slab + MS * 4, o_sjob = o_stgt + MS * 4,

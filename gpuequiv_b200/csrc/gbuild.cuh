@@ -512,14 +512,22 @@ __host__ __device__ __forceinline__ uint32_t node_probe(const View &v, unsigned 
     s = (s + 1) & v.nmask;
   }
 }
+// the set id of a candidate: from SetFillF, or (`stored`) from the table when
+// SetFillF runs in the same pass and checks it there
+__host__ __device__ __forceinline__ uint32_t cand_id(const View &v, uint32_t c, bool stored) {
+  if (!stored) return v.cid[c];
+  const uint32_t id = v.sval[v.cslot[c]];
+  return id < v.sets_cap ? id : 0u;
+}
 struct SuccProbeF {
   View v;
+  bool stored = false;
   __host__ __device__ void operator()(uint32_t s) const {
     Key k = v.succ[s];
     if (k.kind == K_NONE) return;
     if (k.kind != K_CLAUSE) {
-      if (k.a & CAND) k.a = v.cid[k.a & ~CAND];
-      if (k.b & CAND) k.b = v.cid[k.b & ~CAND];
+      if (k.a & CAND) k.a = cand_id(v, k.a & ~CAND, stored);
+      if (k.b & CAND) k.b = cand_id(v, k.b & ~CAND, stored);
       v.succ[s] = k;
     }
     const uint32_t slot = node_probe(v, key_hash(k, v.seed));
@@ -531,16 +539,15 @@ struct SuccProbeF {
     if (v.nval[slot] == UNSET) at_min(&v.nclaim[slot], s);
   }
 };
+// 1 for the slot that numbers a new position
+__host__ __device__ __forceinline__ uint32_t succ_flag(const View &v, uint32_t s) {
+  if (v.succ[s].kind == K_NONE) return 0u;
+  const uint32_t slot = v.sslot[s];
+  return (v.nval[slot] == UNSET && v.nclaim[slot] == s) ? 1u : 0u;
+}
 struct SuccFlagF {
   View v;
-  __host__ __device__ void operator()(uint32_t s) const {
-    uint32_t f = 0;
-    if (v.succ[s].kind != K_NONE) {
-      const uint32_t slot = v.sslot[s];
-      f = (v.nval[slot] == UNSET && v.nclaim[slot] == s) ? 1u : 0u;
-    }
-    v.snew[s] = f;
-  }
+  __host__ __device__ void operator()(uint32_t s) const { v.snew[s] = succ_flag(v, s); }
 };
 struct SuccNewF {
   View v;
@@ -697,6 +704,15 @@ struct RowEndF {
   }
 };
 
+// what level_gate asks, from the level's bounds
+__host__ __device__ __forceinline__ bool level_fits(const View &v, unsigned long long S, unsigned long long E,
+                                                    unsigned long long C) {
+  const unsigned long long nn = v.t[T_NN], ne = v.t[T_NE];
+  const unsigned long long ns = v.ctl->n_sets, top = v.ctl->sdata_top;
+  return S < (1ull << 31) && E < (1ull << 31) && C < (1ull << 31) && S <= v.capS && E <= v.capE && C <= v.capC &&
+         ns + C <= v.sets_cap && top + E <= v.sdata_cap && 2 * (ns + C) <= v.scap && nn + S <= v.nodes_cap &&
+         2 * (nn + S) <= v.ncap && ne + S <= v.edges_cap;
+}
 // ---- level bookkeeping on the device (one thread each) ---------------------------
 // Start of a level: done when the frontier is empty; a frontier beyond the
 // scratch capacity stalls the loop until the host has grown the buffers.
@@ -720,16 +736,9 @@ struct LevelStartF {
 // buffer and table must hold this level, else the level stalls (and is run
 // again after the host grew them).
 __host__ __device__ inline void level_gate(const View &v) {
-  {
-    const unsigned long long S = v.t[T_S], E = v.t[T_E], C = v.t[T_C], nn = v.t[T_NN], ne = v.t[T_NE];
-    const unsigned long long ns = v.ctl->n_sets, top = v.ctl->sdata_top;
-    const bool fits = S < (1ull << 31) && E < (1ull << 31) && C < (1ull << 31) && S <= v.capS && E <= v.capE &&
-                      C <= v.capC && ns + C <= v.sets_cap && top + E <= v.sdata_cap && 2 * (ns + C) <= v.scap &&
-                      nn + S <= v.nodes_cap && 2 * (nn + S) <= v.ncap && ne + S <= v.edges_cap;
-    if (!fits) {
-      v.t[T_GO] = 0;
-      v.t[T_STALL] = 1;
-    }
+  if (!level_fits(v, v.t[T_S], v.t[T_E], v.t[T_C])) {
+    v.t[T_GO] = 0;
+    v.t[T_STALL] = 1;
   }
 }
 struct LevelGateF {
@@ -769,6 +778,19 @@ struct LevelEndF {
 //     (on the device a CUDA graph WHILE node: up to `limit` levels per launch,
 //     stopping as soon as *go == 0).
 //   bool ok();                                             (no backend error so far)
+// A backend with `static constexpr bool kCluster = true` also runs levels with
+// small frontiers in one launch:
+//   bool cluster_ok(uint32_t items);          frontiers of that many positions go there
+//   void cluster_levels(const View &, bool start, uint32_t n_starts);   (start: the start level first)
+//   void cluster_assemble(const View &, const Out &, uint32_t N);  jbase .. jm as after the level loop
+template <class B, class = void>
+struct has_cluster {
+  static constexpr bool value = false;
+};
+template <class B>
+struct has_cluster<B, decltype((void)B::kCluster)> {
+  static constexpr bool value = B::kCluster;
+};
 struct Totals {
   Ctl ctl;
   unsigned long long t[T_COUNT];
@@ -1051,31 +1073,8 @@ class Builder {
     be_.each(1, LevelEndF{v_});
   }
 
-  int attempt_build(const Input &in, unsigned long long seed, Result &out) {
-    v_ = View{};
-    capF_ = capS_ = capE_ = capC_ = capNew_ = capSets_ = capSdata_ = capNodes_ = capEdges_ = scap_ = ncap_ = 0;
-    be_.drop_graph();
-    v_.soff = in.soff;
-    v_.slab = in.slab;
-    v_.stgt = in.stgt;
-    v_.sjob = in.sjob;
-    v_.p0 = in.p0;
-    v_.q0 = in.q0;
-    v_.jsb = in.jsb;
-    v_.heavy_min = in.heavy_min;
-    v_.n_jobs = in.n_jobs;
-    v_.max_pos = in.max_pos;
-    v_.seed = seed;
-    const uint32_t J = in.n_jobs;
-    d_tot_ = get<Totals>(1);
-    v_.jcount = get<uint32_t>(J);
-    v_.jfirst = get<uint32_t>(J);
-    v_.jover = get<uint32_t>(J);
-    if (!d_tot_ || !v_.jcount || !v_.jfirst || !v_.jover) return 1;
-    be_.fill(d_tot_, 0, sizeof(Totals));
-    be_.fill(v_.jcount, 0, (size_t)J * 4);
-    be_.fill(v_.jover, 0, (size_t)J * 4);
-    v_.ctl = &d_tot_->ctl;
+  // The empty set and level 0 as launches of their own.
+  int start_level(const Input &in) {
     // the empty set is set 0
     if (!ensure_sets(0, 0, (uint64_t)in.n_starts + 1, (uint64_t)in.n_starts + 1)) return 1;
     {
@@ -1117,9 +1116,46 @@ class Builder {
     h_tot_.t[T_DONE] = 0;
     h_tot_.t[T_LEVELS] = 0;
     be_.copy(d_tot_, &h_tot_, sizeof(Totals));
+    return 0;
+  }
+
+  int attempt_build(const Input &in, unsigned long long seed, Result &out) {
+    v_ = View{};
+    h_tot_ = Totals{};
+    capF_ = capS_ = capE_ = capC_ = capNew_ = capSets_ = capSdata_ = capNodes_ = capEdges_ = scap_ = ncap_ = 0;
+    be_.drop_graph();
+    v_.soff = in.soff;
+    v_.slab = in.slab;
+    v_.stgt = in.stgt;
+    v_.sjob = in.sjob;
+    v_.p0 = in.p0;
+    v_.q0 = in.q0;
+    v_.jsb = in.jsb;
+    v_.heavy_min = in.heavy_min;
+    v_.n_jobs = in.n_jobs;
+    v_.max_pos = in.max_pos;
+    v_.seed = seed;
+    const uint32_t J = in.n_jobs;
+    d_tot_ = get<Totals>(1);
+    v_.jcount = get<uint32_t>(J);
+    v_.jfirst = get<uint32_t>(J);
+    v_.jover = get<uint32_t>(J);
+    if (!d_tot_ || !v_.jcount || !v_.jfirst || !v_.jover) return 1;
+    be_.fill(d_tot_, 0, sizeof(Totals));
+    be_.fill(v_.jcount, 0, (size_t)J * 4);
+    be_.fill(v_.jover, 0, (size_t)J * 4);
+    v_.ctl = &d_tot_->ctl;
+    const uint32_t T = in.n_starts;
+    bool cluster = false;  // the start level and the first levels in one launch
+    if constexpr (has_cluster<B>::value) cluster = be_.cluster_ok(T);
+    if (!cluster) {
+      const int r = start_level(in);
+      if (r) return r;
+    }
     // first guesses; the gate stalls a level that does not fit and the
     // buffers grow to its exact needs
     {
+      const uint32_t newN = cluster ? T : (uint32_t)h_tot_.t[T_F];
       const uint64_t guess = 8ull * newN + 4096;
       auto mx = [&](uint32_t h) { return (uint32_t)std::max<uint64_t>(guess, h); };
       const uint32_t n_sets = h_tot_.ctl.n_sets, top = h_tot_.ctl.sdata_top;
@@ -1129,12 +1165,13 @@ class Builder {
           ensure_level(mx(hint.S), mx(hint.E), mx(hint.C)) &&
           ensure_sets(n_sets, top, std::max<uint64_t>(guess, hint.sets > n_sets ? hint.sets - n_sets : 0),
                       std::max<uint64_t>(guess, hint.sdata > top ? hint.sdata - top : 0)) &&
-          ensure_nodes(newN, std::max<uint64_t>(guess, hint.nodes > newN ? hint.nodes - newN : 0), 0, mx(hint.edges));
+          ensure_nodes(cluster ? 0 : newN, std::max<uint64_t>(guess, hint.nodes > newN ? hint.nodes - newN : 0), 0,
+                       mx(hint.edges));
       exact_ = false;
       if (!ok)  // the hint asked for more than the device has now: start small
         ok = ensure_frontier(std::max<uint32_t>(newN, 4096)) &&
              ensure_level((uint32_t)guess, (uint32_t)guess, (uint32_t)guess) &&
-             ensure_sets(n_sets, top, guess, guess) && ensure_nodes(newN, guess, 0, guess);
+             ensure_sets(n_sets, top, guess, guess) && ensure_nodes(cluster ? 0 : newN, guess, 0, guess);
       if (!ok) return 1;
       short_ = 0;
     }
@@ -1143,24 +1180,33 @@ class Builder {
     const uint32_t batch = 4096;
     unsigned long long last_stall = ~0ull;
     uint32_t same_stall = 0;
+    bool start = cluster;  // the start level is still to run
     for (;;) {
       sync_view();
-      if (!be_.has_graph()) {
-        be_.begin_capture();
-        enqueue_level();
-        be_.end_capture(tp(T_GO));
-      }
       const unsigned long long levels_before = h_tot_.t[T_LEVELS];
-      be_.run_graph(batch);  // up to `batch` levels, fewer when the loop stops
+      cluster = start;
+      if constexpr (has_cluster<B>::value) {
+        cluster = start || be_.cluster_ok((uint32_t)std::min<unsigned long long>(h_tot_.t[T_F], 0xffffffffull));
+        if (cluster) be_.cluster_levels(v_, start, T);
+      }
+      start = false;
+      if (!cluster) {
+        if (!be_.has_graph()) {
+          be_.begin_capture();
+          enqueue_level();
+          be_.end_capture(tp(T_GO));
+        }
+        be_.run_graph(batch);  // up to `batch` levels, fewer when the loop stops
+      }
       if (!fetch_totals()) return 1;
-      be_.note_levels(h_tot_.t[T_LEVELS] - levels_before + (h_tot_.t[T_STALL] ? 1 : 0));
+      if (!cluster) be_.note_levels(h_tot_.t[T_LEVELS] - levels_before + (h_tot_.t[T_STALL] ? 1 : 0));
       if (h_tot_.ctl.err & ERR_COLLISION) return 3;
       if (h_tot_.ctl.err) return 2;
       if (h_tot_.t[T_DONE]) break;
       if (!h_tot_.t[T_STALL]) {
         // no progress without a stall would be a defect (a recorded loop
         // always runs a level; plain mode runs one as it is "recorded")
-        if (h_tot_.t[T_LEVELS] == levels_before && be_.has_graph()) return 2;
+        if (h_tot_.t[T_LEVELS] == levels_before && !cluster && be_.has_graph()) return 2;
         continue;
       }
       // grow to the stalled level's needs (its bounds were counted, or the
@@ -1185,9 +1231,6 @@ class Builder {
     be_.drop_graph();
     v_.t = d_tot_->t;
     const uint32_t levels = (uint32_t)h_tot_.t[T_LEVELS];
-    if (!fetch_totals()) return 1;
-    if (h_tot_.ctl.err & ERR_COLLISION) return 3;
-    if (h_tot_.ctl.err) return 2;
     // per-job CSR in local ids
     const uint32_t N = (uint32_t)h_tot_.t[T_NN], M = (uint32_t)h_tot_.t[T_NE];
     Out o{};
@@ -1204,11 +1247,18 @@ class Builder {
     if (!o.jbase || !o.fperm || !o.frl || !o.frow || !o.row || !o.rrel || !o.jm || !o.col || !o.wt || !o.att)
       return 1;
     sync_view();
-    be_.scan(v_.jcount, o.jbase, J, &d_tot_->t[T_N]);
-    be_.each(N, PermF{v_, o});
-    be_.scan(o.frl, o.frow, N, &d_tot_->t[T_EDGE]);
-    be_.each(N, RowsF{v_, o});
-    be_.each(J, RowEndF{v_, o});
+    bool assembled = false;
+    if constexpr (has_cluster<B>::value) {
+      assembled = be_.cluster_ok(std::max(N / 8u, J));
+      if (assembled) be_.cluster_assemble(v_, o, N);
+    }
+    if (!assembled) {
+      be_.scan(v_.jcount, o.jbase, J, &d_tot_->t[T_N]);
+      be_.each(N, PermF{v_, o});
+      be_.scan(o.frl, o.frow, N, &d_tot_->t[T_EDGE]);
+      be_.each(N, RowsF{v_, o});
+      be_.each(J, RowEndF{v_, o});
+    }
     if (!fetch_totals()) return 1;
     if (h_tot_.t[T_N] != N || h_tot_.t[T_EDGE] != M || h_tot_.ctl.err) return 2;
     used = Caps{capF_, capS_, capE_, capC_, capSets_, capSdata_, capNodes_, capEdges_};
