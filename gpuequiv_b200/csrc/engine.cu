@@ -2761,6 +2761,8 @@ static geq_status staged_upload(std::vector<CopyJob> &jobs, const char *stage, c
 
 void *Engine::stream_handle() const { return (void *)st->stream; }
 std::shared_ptr<HostPool> Engine::host_pool() const { return st->hpool; }
+void *Engine::pool_get(size_t bytes) { return st->pool.get(bytes); }
+void Engine::pool_put(void *p, size_t bytes) { st->pool.put(p, bytes); }
 
 static geq_status static_scratch(int device, unsigned char *&out);
 static geq_status cluster_setup(uint32_t &blocks);

@@ -727,6 +727,85 @@ __global__ void __launch_bounds__(CLT, 1) k_assemble_cluster(View v, Out o, uint
   cg::this_cluster().sync();
 }
 
+// Signature refinement of a small batch (and the minimised systems) in one
+// launch: five barriers per iteration instead of eight launches and three
+// fills, no read-back to learn whether it converged, and no iteration beyond
+// the one that shows it.
+__global__ void __launch_bounds__(CLT, 1) k_refine_cluster(const rf::Small a) {
+  __shared__ ScanSh sh;
+  const Cluster g = this_cluster_threads();
+  const bool one = g.rank == 0 && threadIdx.x == 0;
+  const uint32_t NS = a.v.NS, J = a.v.J;
+  for (uint32_t i = g.tid; i < NS; i += g.threads) a.part[0][i] = 0u;
+  g.each(J, rf::OneF{a.v.cnt});  // the reference starts from one class (lib.rs:446-448)
+  if (g.rank == 0 && threadIdx.x < 4u) a.flags[threadIdx.x] = 0u;
+  g.sync();
+  uint32_t it = 0, err = 0;
+  rf::RView v = a.v;
+  for (;;) {
+    v.part = a.part[it & 1u];
+    v.npart = a.part[(it + 1u) & 1u];
+    v.isrep = a.isrep[it & 1u];
+    v.rank = a.rank[it & 1u];
+    v.flags = a.flags + 2u * (it & 1u);
+    for (uint32_t i = g.tid; i < a.tab_size; i += g.threads) {
+      v.tab[i] = 0ull;
+      v.claim[i] = UNSET;
+    }
+    g.each(NS, rf::SigF{v});
+    g.sync();
+    if (one) a.flags[2u * ((it + 1u) & 1u)] = 0u;  // the next iteration's; everyone has read it
+    g.each(NS, rf::ProbeF{v});
+    g.sync();
+    g.each(NS, rf::RepF{v});
+    g.sync();
+    {
+      const uint32_t n[1] = {NS};
+      uint32_t *const out[1] = {v.rank};
+      cl_scan<1>(g, n, [&](int, uint32_t i) { return v.isrep[i]; }, out, sh);
+      if (one) *v.tot = sh.tot[0];
+    }
+    g.sync();
+    g.each(NS, rf::AssignF{v});
+    g.each(J, rf::CountJobF{v});
+    g.sync();
+    it++;
+    err = a.flags[1] | a.flags[3];
+    if (err || !v.flags[0] || it > a.max_it) break;
+  }
+  if (a.r.crep && !err) {
+    // the minimised systems in the builder's layout
+    v.part = a.part[it & 1u];
+    {
+      const uint32_t n[1] = {J};
+      uint32_t *const out[1] = {a.cbase};
+      cl_scan<1>(g, n, [&](int, uint32_t i) { return v.cnt[i]; }, out, sh);
+    }
+    const uint32_t NR = (uint32_t)sh.tot[0];
+    if (one) {
+      a.cbase[J] = NR;
+      a.tot[1] = NR;
+    }
+    g.sync();
+    g.each(NS, rf::RepListF{v, a.r});
+    g.sync();
+    {
+      const uint32_t n[1] = {NR};
+      uint32_t *const out[1] = {a.r.roff};
+      cl_scan<1>(g, n, [&](int, uint32_t i) { return a.r.rdeg[i]; }, out, sh);
+    }
+    if (one) {
+      a.r.roff[NR] = (uint32_t)sh.tot[0];
+      a.tot[2] = sh.tot[0];
+    }
+    g.sync();
+    g.each(NR, rf::RowsF{v, a.r});
+    g.each(a.n_starts, rf::MapStartsF{v.part, v.sjob, a.cbase, a.p0, a.q0, a.rp0, a.rq0});
+  }
+  if (one) a.tot[3] = ((unsigned long long)it << 32) | err;
+  cg::this_cluster().sync();
+}
+
 // Backend of the level loop: stream-ordered allocation, kernels and copies on
 // the context's stream.
 struct DevBackend {
@@ -750,8 +829,19 @@ struct DevBackend {
     note(cudaGetLastError());
     return err == cudaSuccess;
   }
+  // Small blocks come from the engine's pool: its blocks go from one user to
+  // the next in the order of this stream, and taking one is no driver call (a
+  // query makes some 80).  Larger ones, whose sizes vary with every build, from
+  // the device's stream-ordered pool.
+  static constexpr size_t POOL_MAX = 4u << 20;
+  Engine *eng = nullptr;
+  std::unordered_map<void *, size_t> pooled;
   void *alloc(size_t b) {
     void *p = nullptr;
+    if (eng && b <= POOL_MAX && (p = eng->pool_get(b)) != nullptr) {
+      pooled.emplace(p, b);
+      return p;
+    }
     cudaError_t e = cudaMallocAsync(&p, b, s);
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -760,15 +850,43 @@ struct DevBackend {
     return p;
   }
   void release(void *p) {
-    if (p) note(cudaFreeAsync(p, s));
+    if (!p) return;
+    auto it = pooled.find(p);
+    if (it == pooled.end()) {
+      note(cudaFreeAsync(p, s));
+      return;
+    }
+    eng->pool_put(p, it->second);
+    pooled.erase(it);
   }
   void fill(void *p, int v, size_t b) { note(cudaMemsetAsync(p, v, b, s)); }
   void copy(void *d, const void *src, size_t b) {
     if (b) note(cudaMemcpyAsync(d, src, b, cudaMemcpyDefault, s));
   }
-  void fetch(void *h, const void *d, size_t b) {
-    copy(h, d, b);
+  // small read-backs go through page-locked memory: a copy to pageable memory
+  // is a wait of its own
+  HostBuf bounce;
+  static constexpr size_t BOUNCE = 64u << 10;
+  void fetch(void *h, const void *d, size_t b) { fetch3(h, d, b, nullptr, nullptr, 0, nullptr, nullptr, 0); }
+  void fetch3(void *h0, const void *d0, size_t b0, void *h1, const void *d1, size_t b1, void *h2, const void *d2,
+              size_t b2) {
+    void *h[3] = {h0, h1, h2};
+    const void *d[3] = {d0, d1, d2};
+    const size_t b[3] = {b0, b1, b2};
+    char *at[3] = {nullptr, nullptr, nullptr};
+    size_t o = 0;
+    for (int k = 0; k < 3; k++) {
+      if (!b[k]) continue;
+      const size_t n = (b[k] + 15) & ~(size_t)15;
+      if (o + n <= BOUNCE && eng && (bounce.p || bounce.alloc(eng->host_pool(), BOUNCE)) && bounce.pool) {
+        at[k] = (char *)bounce.p + o;
+        o += n;
+      }
+      copy(at[k] ? at[k] : h[k], d[k], b[k]);
+    }
     note(cudaStreamSynchronize(s));
+    for (int k = 0; k < 3; k++)
+      if (at[k]) std::memcpy(h[k], at[k], b[k]);
   }
   template <class F>
   void each(uint32_t n, const F &f) {
@@ -930,6 +1048,11 @@ struct DevBackend {
   void cluster_levels(const View &v, bool start, uint32_t n_starts) {
     launch_cluster(k_levels_cluster, CL_SMEM, v, start ? 1u : 0u, n_starts, CL_FRONTIER);
   }
+  // one thread per state and per job, twice over at most
+  bool cluster_refine_ok(uint32_t states, uint32_t jobs) const {
+    return cluster_blocks && !plain && states <= 2 * 16 * CLT && jobs <= 2 * 16 * CLT;
+  }
+  void cluster_refine(const rf::Small &a) { launch_cluster(k_refine_cluster, 0, a); }
   void cluster_assemble(const View &v, const Out &o, uint32_t N) { launch_cluster(k_assemble_cluster, 0, v, o, N); }
   // Sets the kernels up on the current device; the blocks of a cluster, 0 when
   // even 8 do not fit.
@@ -939,7 +1062,8 @@ struct DevBackend {
       if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
       return e;
     };
-    if (attrs(k_levels_cluster, CL_SMEM) != cudaSuccess || attrs(k_assemble_cluster, 0) != cudaSuccess) {
+    if (attrs(k_levels_cluster, CL_SMEM) != cudaSuccess || attrs(k_assemble_cluster, 0) != cudaSuccess ||
+        attrs(k_refine_cluster, 0) != cudaSuccess) {
       cudaGetLastError();
       return 0;
     }
@@ -971,10 +1095,8 @@ struct DevBackend {
   }
   ~DevBackend() {
     drop_graph();
-    if (d_loop) cudaFreeAsync(d_loop, s);
-    if (part) cudaFreeAsync(part, s);
-    for (void *q : {(void *)lb_ctl, (void *)lb_flag, (void *)lb_agg, (void *)lb_inc})
-      if (q) cudaFreeAsync(q, s);
+    for (void *q : {(void *)d_loop, (void *)part, (void *)lb_ctl, (void *)lb_flag, (void *)lb_agg, (void *)lb_inc})
+      release(q);
   }
 };
 
@@ -1052,6 +1174,7 @@ static geq_status device_build(Engine &eng, int device, uint32_t n_jobs, const L
       cudaGetLastError();
     });
   gb::DevBackend &be = db.be;
+  be.eng = &eng;
   be.s = (cudaStream_t)eng.stream_handle();
   be.n_sms = eng.n_sms;
   // GEQ_TUNE_NO_GRAPH: levels as plain launches (ncu does not profile the
@@ -1115,15 +1238,11 @@ static geq_status device_build(Engine &eng, int device, uint32_t n_jobs, const L
   if (trivial) {
     const auto tm = clk::now();
     db.rf.reset(new rf::Refiner<gb::DevBackend>(be));
-    int rrc = db.rf->run(in);
-    uint32_t *rp0 = nullptr, *rq0 = nullptr;
-    if (rrc == 0) rrc = db.rf->reduce(in, bin, rp0, rq0);
+    // the bisimilar short cut is decided on the host from the mapped starts
+    std::vector<uint32_t> mp((size_t)T), mq((size_t)T);
+    const int rrc = db.rf->run_reduce(in, bin, mp.data(), mq.data());
     geq_status rst = refine_status(rrc, be);
     if (rst) return rst;
-    // the bisimilar short cut, decided on the host from the mapped starts
-    std::vector<uint32_t> mp((size_t)T), mq((size_t)T);
-    be.copy(mp.data(), rp0, (size_t)T * 4);
-    be.fetch(mq.data(), rq0, (size_t)T * 4);
     if (!be.ok()) return fail(GEQ_ERR_CUDA, "device minimisation: %s", cudaGetErrorString(be.err));
     trivial->assign(n_jobs, 0);
     std::vector<uint32_t> keep;
@@ -1137,34 +1256,40 @@ static geq_status device_build(Engine &eng, int device, uint32_t n_jobs, const L
       for (uint32_t t = t0j; t < t1j; t++) keep.push_back(t);
     }
     const uint32_t K = (uint32_t)keep.size();
-    std::vector<uint32_t> hst(2 * (size_t)K + 1);
-    for (uint32_t k = 0; k < K; k++) {
-      hst[k] = mp[keep[k]];
-      hst[K + k] = mq[keep[k]];
+    if (K != T) {  // else the mapped starts as they are on the device
+      std::vector<uint32_t> hst(2 * (size_t)K + 1);
+      for (uint32_t k = 0; k < K; k++) {
+        hst[k] = mp[keep[k]];
+        hst[K + k] = mq[keep[k]];
+      }
+      db.dstarts = (uint32_t *)be.alloc(((size_t)2 * K + 1) * 4);
+      if (!db.dstarts) return fail(GEQ_ERR_OUT_OF_MEMORY, "device start positions");
+      be.copy(db.dstarts, hst.data(), ((size_t)2 * K + 1) * 4);
+      bin.p0 = db.dstarts;
+      bin.q0 = db.dstarts + K;
+      bin.n_starts = K;
+      be.fetch(hst.data(), db.dstarts, 4);  // the host copy above is done
     }
-    db.dstarts = (uint32_t *)be.alloc(((size_t)2 * K + 1) * 4);
-    if (!db.dstarts) return fail(GEQ_ERR_OUT_OF_MEMORY, "device start positions");
-    be.copy(db.dstarts, hst.data(), ((size_t)2 * K + 1) * 4);
-    bin.p0 = db.dstarts;
-    bin.q0 = db.dstarts + K;
-    bin.n_starts = K;
-    be.fetch(hst.data(), db.dstarts, 4);  // the host copy above is done
     db.minimize_ms = std::chrono::duration<double, std::milli>(clk::now() - tm).count();
   }
   const auto t1 = clk::now();
   db.b.reset(new gb::Builder<gb::DevBackend>(be));
-  // start from the capacities the previous build on this stream ended with
+  // start from the capacities the previous build of about as many start
+  // positions on this stream ended with (one hint for all sizes made a single
+  // query after a batch clear the batch's hash tables: equivalences() of a
+  // 40-state system 3.3 against 2.8 ms)
   static std::mutex hint_mu;
-  static std::unordered_map<void *, gb::Builder<gb::DevBackend>::Caps> hints;
+  static std::map<std::pair<void *, uint32_t>, gb::Builder<gb::DevBackend>::Caps> hints;
+  const std::pair<void *, uint32_t> hint_key((void *)be.s, 32u - lzcnt32(bin.n_starts));
   {
     std::lock_guard<std::mutex> g(hint_mu);
-    auto it = hints.find((void *)be.s);
+    auto it = hints.find(hint_key);
     if (it != hints.end()) db.b->hint = it->second;
   }
   const int rc = db.b->run(bin, db.r);
   if (rc == 0) {
     std::lock_guard<std::mutex> g(hint_mu);
-    hints[(void *)be.s] = db.b->used;
+    hints[hint_key] = db.b->used;
   }
   db.upload_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
   db.build_ms = std::chrono::duration<double, std::milli>(clk::now() - t1).count();
@@ -1194,9 +1319,8 @@ geq_status build_and_upload(Engine &eng, int device, uint32_t n_jobs, const Lts 
   geq_status st = device_build(eng, device, n_jobs, L, start_off, p, q, max_positions, db, trivial);
   if (st) return st;
   std::vector<uint32_t> jcount(n_jobs), jm(n_jobs), jover(n_jobs);
-  db.be.copy(jcount.data(), db.r.jcount, (size_t)n_jobs * 4);
-  db.be.copy(jover.data(), db.r.jover, (size_t)n_jobs * 4);
-  db.be.fetch(jm.data(), db.r.jm, (size_t)n_jobs * 4);
+  db.be.fetch3(jcount.data(), db.r.jcount, (size_t)n_jobs * 4, jover.data(), db.r.jover, (size_t)n_jobs * 4, jm.data(),
+               db.r.jm, (size_t)n_jobs * 4);
   if (!db.be.ok()) return fail(GEQ_ERR_CUDA, "device game build: %s", cudaGetErrorString(db.be.err));
   if (over) over->assign(n_jobs, 0);
   for (uint32_t j = 0; j < n_jobs; j++) {

@@ -783,6 +783,8 @@ struct LevelEndF {
 //   bool cluster_ok(uint32_t items);          frontiers of that many positions go there
 //   void cluster_levels(const View &, bool start, uint32_t n_starts);   (start: the start level first)
 //   void cluster_assemble(const View &, const Out &, uint32_t N);  jbase .. jm as after the level loop
+//   bool cluster_refine_ok(uint32_t states, uint32_t jobs); void cluster_refine(const rf::Small &);  (refine.cuh)
+//   void fetch3(h0, d0, b0, h1, d1, b1, h2, d2, b2);  three fetches and one wait
 template <class B, class = void>
 struct has_cluster {
   static constexpr bool value = false;

@@ -260,6 +260,9 @@ class Engine {
   // the other device passes of the library (the device game builder).
   void *stream_handle() const;
   std::shared_ptr<HostPool> host_pool() const;
+  // Device blocks from the engine's pool, for users of the engine's stream.
+  void *pool_get(size_t bytes);
+  void pool_put(void *p, size_t bytes);
   geq_tuning tuning{};
   int n_sms = 0;
   uint64_t total_mem = 0;

@@ -215,6 +215,24 @@ struct MapStartsF {
   }
 };
 
+// The whole minimisation of a small batch in one launch (a backend with
+// kCluster): the two buffers of each alternating array, and the minimised
+// systems' arrays when they are wanted (r.crep set; room for NS states and MS
+// transitions).  out: iterations run, representatives, transitions kept.
+struct Small {
+  RView v;
+  uint32_t *part[2], *isrep[2], *rank[2];
+  uint32_t tab_size;
+  uint32_t max_it;
+  Reduce r;
+  uint32_t *cbase;
+  const uint32_t *p0, *q0;
+  uint32_t *rp0, *rq0;
+  uint32_t n_starts;
+  uint32_t *flags;            // two pairs [changed, error]
+  unsigned long long *tot;    // [0] scan total, [1] states, [2] transitions, [3] iterations << 32 | error
+};
+
 // Host driver over the same backend interface as gb::Builder.
 template <class B>
 class Refiner {
@@ -223,12 +241,50 @@ class Refiner {
   ~Refiner() { release_all(); }
   // 0 ok; 1 out of memory / backend failure; 3 repeated fingerprint collisions
   int run(const gb::Input &in) {
+    small_ = false;
+    if constexpr (gb::has_cluster<B>::value) {
+      if (be_.cluster_refine_ok(in.NS, in.n_jobs)) {
+        for (uint32_t attempt = 0; attempt < 4; attempt++) {
+          const int r = small_run(in, seed_of(attempt), false);
+          if (r != 3) return r;
+          release_all();
+        }
+        return 3;
+      }
+    }
     for (uint32_t attempt = 0; attempt < 4; attempt++) {
-      const int r = attempt_run(in, 0x13198a2e03707344ull + 0x9e3779b97f4a7c15ull * attempt);
+      const int r = attempt_run(in, seed_of(attempt));
       if (r != 3) return r;
       release_all();
     }
     return 3;
+  }
+  // run() and reduce() together; the mapped start positions go to the host
+  // arrays h_p0 / h_q0 (in.n_starts each) as well.
+  int run_reduce(const gb::Input &in, gb::Input &out, uint32_t *h_p0, uint32_t *h_q0) {
+    uint32_t *rp0 = nullptr, *rq0 = nullptr;
+    const size_t tb = (size_t)in.n_starts * 4;
+    if constexpr (gb::has_cluster<B>::value) {
+      if (be_.cluster_refine_ok(in.NS, std::max(in.n_jobs, in.n_starts))) {
+        for (uint32_t attempt = 0; attempt < 4; attempt++) {
+          const int r = small_run(in, seed_of(attempt), true, h_p0, h_q0);
+          if (r == 3) {
+            release_all();
+            continue;
+          }
+          if (r) return r;
+          reduced(in, sm_.r, sm_.cbase, sm_.rp0, sm_.rq0, out);
+          return 0;
+        }
+        return 3;
+      }
+    }
+    int r = run(in);
+    if (!r) r = reduce(in, out, rp0, rq0);
+    if (r) return r;
+    be_.copy(h_p0, rp0, tb);
+    be_.fetch(h_q0, rq0, tb);
+    return be_.ok() ? 0 : 1;
   }
   uint32_t iterations = 0;
   const uint32_t *partition() const { return final_; }  // per state: job-local class
@@ -270,16 +326,7 @@ class Refiner {
     if (!r.rlab || !r.rtgt) return 1;
     be_.each(NR, RowsF{v, r});
     be_.each(T, MapStartsF{final_, in.sjob, cbase, in.p0, in.q0, rp0, rq0});
-    out = in;
-    out.NS = NR;
-    out.MS = MR;
-    out.soff = r.roff;
-    out.slab = r.rlab;
-    out.stgt = r.rtgt;
-    out.sjob = r.rjob;
-    out.jsb = cbase;
-    out.p0 = rp0;
-    out.q0 = rq0;
+    reduced(in, r, cbase, rp0, rq0, out);
     be_.fetch(htot_, tot_, sizeof(htot_));  // the host copies above are done
     return be_.ok() ? 0 : 1;
   }
@@ -292,6 +339,104 @@ class Refiner {
   unsigned long long htot_[4] = {0, 0, 0, 0};
   uint32_t hflags_[2] = {0, 0};
   const uint32_t *final_ = nullptr;
+  Small sm_{};
+  bool small_ = false;
+  static unsigned long long seed_of(uint32_t attempt) {
+    return 0x13198a2e03707344ull + 0x9e3779b97f4a7c15ull * attempt;
+  }
+  static void reduced(const gb::Input &in, const Reduce &r, const uint32_t *cbase, const uint32_t *rp0,
+                      const uint32_t *rq0, gb::Input &out) {
+    out = in;
+    out.NS = r.NR;
+    out.MS = r.MR;
+    out.soff = r.roff;
+    out.slab = r.rlab;
+    out.stgt = r.rtgt;
+    out.sjob = r.rjob;
+    out.jsb = cbase;
+    out.p0 = rp0;
+    out.q0 = rq0;
+  }
+  // One launch for all iterations (and the minimised systems); 3: a
+  // fingerprint collision.
+  int small_run(const gb::Input &in, unsigned long long seed, bool reduce, uint32_t *h_p0 = nullptr,
+                uint32_t *h_q0 = nullptr) {
+    const uint32_t NS = in.NS, J = in.n_jobs, T = reduce ? in.n_starts : 0u;
+    uint64_t cap = 1024;
+    while (cap < 4 * (uint64_t)NS) cap <<= 1;
+    // one block: 8-byte arrays first
+    size_t words = 0;
+    auto take = [&](size_t n) {
+      const size_t o = words;
+      words += (n + 1) & ~(size_t)1;
+      return o;
+    };
+    const size_t o_sig = take(2 * (size_t)in.MS), o_fp = take(2 * (size_t)NS), o_tab = take(2 * cap), o_tot = take(8),
+                 o_claim = take(cap), o_part = take(2 * (size_t)NS), o_isrep = take(2 * (size_t)NS),
+                 o_rank = take(2 * (size_t)NS), o_slen = take(NS), o_slot = take(NS), o_rep = take(NS),
+                 o_cnt = take(J), o_flags = take(4);
+    const size_t o_cbase = take(reduce ? (size_t)J + 1 : 0), o_crep = take(reduce ? NS : 0),
+                 o_rdeg = take(reduce ? NS : 0), o_roff = take(reduce ? (size_t)NS + 1 : 0),
+                 o_rjob = take(reduce ? NS : 0), o_rlab = take(reduce ? in.MS : 0), o_rtgt = take(reduce ? in.MS : 0),
+                 o_rp0 = take(T), o_rq0 = take(T);
+    uint32_t *w = get<uint32_t>(words);
+    if (!w) return 1;
+    Small &s = sm_;
+    s = Small{};
+    RView &v = s.v;
+    v.soff = in.soff;
+    v.slab = in.slab;
+    v.stgt = in.stgt;
+    v.sjob = in.sjob;
+    v.jsb = in.jsb;
+    v.NS = NS;
+    v.J = J;
+    v.seed = seed;
+    v.mask = (uint32_t)cap - 1;
+    v.sig = (unsigned long long *)(w + o_sig);
+    v.fp = (unsigned long long *)(w + o_fp);
+    v.tab = (unsigned long long *)(w + o_tab);
+    v.tot = s.tot = (unsigned long long *)(w + o_tot);
+    v.claim = w + o_claim;
+    v.slen = w + o_slen;
+    v.slot = w + o_slot;
+    v.rep = w + o_rep;
+    v.cnt = w + o_cnt;
+    s.flags = w + o_flags;
+    for (int k = 0; k < 2; k++) {
+      s.part[k] = w + o_part + (size_t)k * NS;
+      s.isrep[k] = w + o_isrep + (size_t)k * NS;
+      s.rank[k] = w + o_rank + (size_t)k * NS;
+    }
+    s.tab_size = (uint32_t)cap;
+    s.max_it = NS + 2;
+    if (reduce) {
+      s.cbase = w + o_cbase;
+      s.r = Reduce{s.cbase, w + o_crep, w + o_rdeg, w + o_roff, (int32_t *)(w + o_rlab), w + o_rtgt, w + o_rjob, NS,
+                   in.MS};
+      s.p0 = in.p0;
+      s.q0 = in.q0;
+      s.rp0 = w + o_rp0;
+      s.rq0 = w + o_rq0;
+      s.n_starts = T;
+    }
+    be_.cluster_refine(s);
+    be_.fetch3(htot_, s.tot, sizeof(htot_), h_p0, s.rp0, (size_t)T * 4, h_q0, s.rq0, (size_t)T * 4);
+    if (!be_.ok()) return 1;
+    const uint32_t err = (uint32_t)htot_[3];
+    if (err & 1u) return 3;
+    if (err) return 1;
+    iterations = (uint32_t)(htot_[3] >> 32);
+    s.r.NR = (uint32_t)htot_[1];
+    s.r.MR = (uint32_t)htot_[2];
+    v_ = v;
+    tot_ = s.tot;
+    final_ = s.part[iterations & 1];
+    final_isrep_ = s.isrep[(iterations - 1) & 1];
+    final_rank_ = s.rank[(iterations - 1) & 1];
+    small_ = true;
+    return 0;
+  }
   uint32_t *final_isrep_ = nullptr, *final_rank_ = nullptr;
   template <class T>
   T *get(size_t n) {
