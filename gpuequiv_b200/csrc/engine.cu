@@ -107,6 +107,8 @@ struct Ctr {
   uint32_t next_slot;  // k_round: next frontier slot to hand out (32 per grab)
   uint32_t nbig;       // large positions queued by k_round for k_round_big
   uint32_t next_big;   // k_round_big: next queue entry to hand out
+  uint32_t npush;      // parts of long predecessor lists queued for k_round_big
+  uint32_t next_push;  // k_round_big: next of them to hand out
   uint32_t pad3;
   unsigned long long positions, edges, bytes, rounds;
 #if GEQ_PATH_PROFILE
@@ -152,6 +154,9 @@ struct KParams {
   uint32_t fblocks;      // blocks of k_commit, k_fcount, k_ffill
   const uint32_t *abits; // attacker positions as a bitmap (mwords words)
   uint32_t *bigq;        // frontier slots of the large positions of the round
+  // parts of long predecessor lists (first entry | entries << 32 | changed
+  // from empty << 63); null: a warp pushes its positions' lists itself
+  unsigned long long *pushq;
   // edge pairs for the lane path: successor id (low word) and the update in
   // the codec's pack_edge form (high word); null: read col / wt
   const unsigned long long *cw;
@@ -1549,18 +1554,57 @@ __device__ __forceinline__ void push_one(const KParams &p, uint32_t u, uint32_t 
   mark_push(p, u, stamp);
 }
 
+// Predecessors rcol[b, b+n) into the next frontier by the whole warp, four a
+// lane at a time so that their loads overlap.
+__device__ __forceinline__ void push_run(const KParams &p, Ctr *c, uint32_t b, uint32_t n, uint32_t stamp,
+                                         uint32_t lane, bool first) {
+  for (uint32_t t0 = 0; t0 < n; t0 += 128u) {
+    uint32_t u[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t t = t0 + (uint32_t)k * 32u + lane;
+      u[k] = t < n ? ld(p.rcol, (unsigned long long)b + t, p.n_edges, c) : ~0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (t0 + (uint32_t)k * 32u + lane < n && CHECK_IDX(c, u[k], p.n_nodes)) push_one(p, u[k], stamp, first);
+  }
+}
+
 // Put the predecessors of the flagged lanes' positions into the next
-// frontier.  The reverse-CSR ranges of all flagged lanes are concatenated and
-// walked 32 entries at a time, so a position with many predecessors is spread
-// over the whole warp.
+// frontier.  A list of PUSH_LONG entries or more is queued in parts for all
+// warps of k_round_big (`queue`): in-degrees reach tens of thousands, such
+// positions sit side by side, and the warp that met them all would be the
+// round's length.  One of PUSH_RUN or more is walked by the warp on its own;
+// the other ranges are concatenated and walked 32 entries at a time.
+// Measured on one B200: rounds of a 125,000-position game whose clauses have
+// 17,000-30,000 predecessors 8.96 -> 0.61 ms of k_round (the call 13.0 -> 4.6
+// ms), 1,400 games resident 17.2 -> 14.9 ms; PUSH_LONG at 256 to 4,096 and
+// PUSH_RUN at 32 to 200 differ by less than the runs do.
+constexpr uint32_t PUSH_RUN = 64, PUSH_LONG = 512;
 __device__ void push_preds_warp(const KParams &p, Ctr *c, uint32_t *sm, uint32_t v, bool flagged, uint32_t stamp,
-                                uint32_t lane, bool first = false) {
+                                uint32_t lane, bool first = false, bool queue = false) {
   const uint32_t firsts = __ballot_sync(FULL, flagged && first);
   uint32_t b = 0, n = 0;
   if (flagged) {
     b = ld(p.rrow, v, p.n_nodes + 1, c);
     n = ld(p.rrow, (unsigned long long)v + 1, p.n_nodes + 1, c) - b;
   }
+  if (queue && p.pushq && n >= PUSH_LONG) {
+    const uint32_t parts = (n + PUSH_LONG - 1u) / PUSH_LONG;
+    const uint32_t at = atomicAdd(&c->npush, parts);
+    for (uint32_t k = 0; k < parts; k++)
+      if (CHECK_IDX(c, at + k, p.n_edges / (PUSH_LONG / 2u) + 1u))
+        p.pushq[at + k] = (unsigned long long)(b + k * PUSH_LONG) |
+                          ((unsigned long long)min(PUSH_LONG, n - k * PUSH_LONG) << 32) |
+                          (first ? 1ull << 63 : 0ull);
+    n = 0;
+  }
+  for (uint32_t m = __ballot_sync(FULL, n >= PUSH_RUN); m; m &= m - 1u) {
+    const uint32_t l = (uint32_t)__ffs((int)m) - 1u;
+    push_run(p, c, __shfl_sync(FULL, b, l), __shfl_sync(FULL, n, l), stamp, lane, (firsts >> l) & 1u);
+  }
+  if (n >= PUSH_RUN) n = 0;
   const uint32_t incl = warp_incl_scan(n, lane);
   const uint32_t total = __shfl_sync(FULL, incl, 31);
   if (total == 0u) return;
@@ -1583,6 +1627,11 @@ __device__ void push_preds_warp(const KParams &p, Ctr *c, uint32_t *sm, uint32_t
     }
   }
   __syncwarp();
+}
+// Entry i of the queue of parts.
+__device__ __forceinline__ void push_part(const KParams &p, Ctr *c, uint32_t i, uint32_t stamp, uint32_t lane) {
+  const unsigned long long e = ld(p.pushq, i, p.n_edges / (PUSH_LONG / 2u) + 1u, c);
+  push_run(p, c, (uint32_t)e, (uint32_t)(e >> 32) & 0x7FFFFFFFu, stamp, lane, (e >> 63) != 0ull);
 }
 
 template <class Cd, int MINB>
@@ -1688,7 +1737,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_round(const KParams p) {
       }
     }
 #endif
-    push_preds_warp(p, c, sm, v, ts == T_CHANGED, stamp, lane, old_cnt == 0u);
+    push_preds_warp(p, c, sm, v, ts == T_CHANGED, stamp, lane, old_cnt == 0u, true);
     if (ts == T_OVERFLOW) mark_push(p, v, stamp);
 #if GEQ_PATH_PROFILE
     if (lane == 0) PROF_ADD(PF_CYC_PUSH, clock64() - tq1);
@@ -1727,8 +1776,8 @@ __global__ void __launch_bounds__(BLOCK, GEQ_BIG_BLOCKS_PER_SM) k_round_big(cons
   __shared__ uint32_t tscr[WARPS_PER_BLOCK * TSCR * 32];
   Ctr *c = p.ctr;
   if (c->halt) return;
-  const uint32_t nb = c->nbig;
-  if (nb == 0) return;
+  const uint32_t nb = c->nbig, np = c->npush;
+  if (nb == 0 && np == 0) return;
   const uint32_t cur = c->cur;
   const uint32_t *F = cur ? p.front1 : p.front0;
   const uint32_t stamp = c->stamp + 1u;
@@ -1744,6 +1793,15 @@ __global__ void __launch_bounds__(BLOCK, GEQ_BIG_BLOCKS_PER_SM) k_round_big(cons
 #if GEQ_PATH_PROFILE
   const long long t0 = clock64();
 #endif
+  if (np) {
+    for (;;) {
+      uint32_t i = 0;
+      if (lane == 0) i = atomicAdd(&c->next_push, 1u);
+      i = __shfl_sync(FULL, i, 0);
+      if (i >= np) break;
+      push_part(p, c, i, stamp, lane);
+    }
+  }
   for (;;) {
     uint32_t i = 0;
     if (lane == 0) i = atomicAdd(&c->next_big, 1u);
@@ -1959,6 +2017,8 @@ __global__ void k_ffill(const KParams p) {
     c->next_slot = 0u;
     c->nbig = 0u;
     c->next_big = 0u;
+    c->npush = 0u;
+    c->next_push = 0u;
     if (c->overflow) c->halt = 1u;
   }
 }
@@ -2575,6 +2635,7 @@ struct DeviceGamesImpl {
   uint32_t *missing = nullptr, *missing_init = nullptr;  // defenders: successors with no energies yet
   std::vector<unsigned long long> off_ranges;  // position ranges of games that are not solved (pairs)
   uint32_t *mark = nullptr, *front0 = nullptr, *front1 = nullptr, *fpart = nullptr, *abits = nullptr, *bigq = nullptr;
+  unsigned long long *pushq = nullptr;
   uint32_t *init_data = nullptr;
   unsigned long long init_total = 0;
   char *inbuf = nullptr;  // row, col, wt, flags, reach, init_data, [desc_init], node bases
@@ -3170,7 +3231,7 @@ geq_status Engine::alloc_work(DeviceGamesImpl &D, bool any_init) {
       (!any_init && !D.alloc(D.desc_init, N)) || !D.alloc(D.slot_new, N) || !D.alloc(D.mark, 2 * ((N + 31) / 32)) ||
       !D.alloc(D.front0, N) || !D.alloc(D.front1, N) || !D.alloc(D.ctr, 1) ||
       !D.alloc(D.fpart, 2 * (size_t)std::max(1, n_sms * GEQ_FRONTIER_BLOCKS_PER_SM)) || !D.alloc(D.abits, (N + 31) / 32) ||
-      !D.alloc(D.bigq, N) || !D.alloc(D.cw, M))
+      !D.alloc(D.bigq, N) || !D.alloc(D.cw, M) || !D.alloc(D.pushq, M / (PUSH_LONG / 2) + 1))
     return fail(GEQ_ERR_OUT_OF_MEMORY, "device allocation for %llu positions / %llu edges failed", N, M);
   unsigned long long cap = std::max<unsigned long long>(4ull * (D.init_total + N) + (1ull << 20), 1ull << 22);
   if (!D.alloc(D.arena[0], cap)) return fail(GEQ_ERR_OUT_OF_MEMORY, "energy arena of %llu words", cap);
@@ -3250,6 +3311,7 @@ geq_status Engine::finish_upload(GamesPtr &dg, bool any_init, GamesPtr &out) {
       1, std::min<unsigned long long>((unsigned long long)n_sms * GEQ_FRONTIER_BLOCKS_PER_SM, (N + 511) / 512));
   kp.abits = D.abits;
   kp.bigq = D.bigq;
+  kp.pushq = D.pushq;
   kp.cw = D.cw;
   kp.missing = nullptr;
   kp.el = D.conf.elements; kp.mx = D.conf.max; kp.eb = D.conf.energy_bits(); kp.em = D.conf.energy_mask();
@@ -4183,10 +4245,18 @@ __device__ void group_rounds(const KParams &p, Ctr *c, const Group &g, RoundStat
           old_cnt = was_empty ? 0u : 1u;
         }
       }
-      push_preds_warp(p, c, sm, v, changed, stamp, lane, old_cnt == 0u);
+      push_preds_warp(p, c, sm, v, changed, stamp, lane, old_cnt == 0u, true);
       if (retry) mark_push(p, v, stamp);  // again after the arena was compacted
     }
     g.sync();
+    if (p.pushq) {
+      const uint32_t np = *(volatile uint32_t *)&c->npush;
+      if (np) {
+        for (uint32_t i = gw; i < np; i += warps) push_part(p, c, i, stamp, lane);
+        g.sync();
+        if (g.tid == 0) c->npush = 0u;  // the next round's warps add to it behind the barrier below
+      }
+    }
     uint32_t *clear = p.mark + (st.stamp & 1u) * p.mwords;
     for (uint32_t i = g.tid; i < p.mwords; i += g.threads) clear[i] = 0u;
     for (uint32_t s2 = g.tid; s2 < st.fs; s2 += g.threads) {
@@ -4241,6 +4311,8 @@ __global__ void __launch_bounds__(CT, 1) k_rounds_cluster(const KParams p, uint3
     c->next_slot = 0u;
     c->nbig = 0u;
     c->next_big = 0u;
+    c->npush = 0u;
+    c->next_push = 0u;
     if (c->overflow) c->halt = 1u;
   }
 }

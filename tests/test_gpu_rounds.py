@@ -118,6 +118,36 @@ def test_launch_forms(geq, ctx, n, form):
         assert canon(d[int(o[v]):int(o[v + 1])]) == canon(exp[v]), f"position {v}"
 
 
+@pytest.mark.parametrize("n", [30_000, 60_000])
+@pytest.mark.parametrize("indeg", [63, 64, 511, 512, 513, 20_000])
+def test_long_predecessor_lists(geq, ctx, n, indeg):
+    """Positions with as many predecessors as the lines between the ways to
+    push them, many of them side by side, inside one launch (30,000 positions)
+    and as rounds of kernels (60,000)."""
+    rng = np.random.default_rng(indeg)
+    hubs = 12  # defenders without successors, each reached by `indeg` attackers
+    srcs = np.concatenate([np.sort(rng.choice(np.arange(hubs, n), indeg, replace=False)) for _ in range(hubs)])
+    dst = np.repeat(np.arange(hubs), indeg)
+    extra_s = np.arange(hubs, n)  # and a chain, so that the pushes go on
+    src = np.concatenate([srcs, extra_s]).astype(np.int64)
+    dst = np.concatenate([dst, np.concatenate([extra_s[1:], [hubs]])])
+    order = np.argsort(src, kind="stable")
+    src, dst = src[order], dst[order].astype(np.uint32)
+    row = np.zeros(n + 1, np.uint32)
+    row[1:] = np.cumsum(np.bincount(src, minlength=n))
+    wt = (np.uint32(1) << (4 * rng.integers(0, N_EL, len(src))).astype(np.uint32)).astype(np.uint32)
+    att = np.ones(n, np.uint8)
+    att[:hubs] = 0
+    g = geq.GameGraph.from_csr(row, dst, wt, att, geq.EnergyConf.STANDARD)
+    offs, data, _ = geq.run_batch_raw([g], ctx)
+    o, d = offs[0].astype(np.int64), data[0]
+    exp = ora.run_game(6, 3, row, dst, wt, att, ora.standard_reach(row, att))
+    lists = exp.lists()
+    assert np.array_equal(np.diff(o), [len(x) for x in lists])
+    for v in range(n):
+        assert canon(d[o[v]:o[v + 1]]) == canon(lists[v]), f"position {v}"
+
+
 @pytest.mark.parametrize("seed,n,mean_deg,merges", [(1, 6000, 3.0, 1), (2, 9000, 1.6, 2), (3, 5000, 7.0, 3),
                                                     (4, 7000, 2.5, 0)])
 def test_small_and_large_rounds_agree(geq, ctx, seed, n, mean_deg, merges):
