@@ -19,16 +19,19 @@
 // the next frontier (a bitmap turned into a list).
 //
 // One warp per frontier position.  A position's new list is built as an
-// antichain in the warp's slice of a global scratch: each candidate (an
-// inverse-updated successor energy, a supremum) is tested against the
-// members by the 32 lanes at once and either dropped or inserted while the
-// members it dominates are removed.  Field-wise <= and max run word by word
+// antichain: of energies of one, two or four words in shared memory, 32
+// candidates (inverse-updated successor energies, suprema) at a time
+// (insert32); of others, and beyond 256 members, in the warp's slice of a
+// global scratch, where each candidate is tested against the members by the 32
+// lanes at once and either dropped or inserted while the members it dominates
+// are removed.  Field-wise <= and max run word by word
 // with SWAR arithmetic (fields of 1-16 bits in guarded 2k-bit slots; 32-bit
 // fields directly).  A position whose antichain outgrows its scratch is
 // recorded and computed again in the same round with a larger scratch; a
 // round whose results outgrow the arena is run again after the arena has
 // been compacted and grown.  Either way only committed lists are read, so a
 // repeated computation gives the same lists.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <chrono>
@@ -50,11 +53,14 @@ constexpr unsigned long long CNT_MASK = (1ull << CNT_BITS) - 1ull;
 
 struct Ctr {
   unsigned long long arena_top;  // energies in use
+  unsigned long long rounds;     // completed by k_wide_cluster
   unsigned long long positions, edges, bytes;
   uint32_t next_slot;   // slots handed out to warps
   uint32_t n_ovf;       // slots whose antichain outgrew the warp scratch
   uint32_t arena_full;  // a new list found no arena space
   uint32_t next_size;   // size of the next frontier
+  uint32_t flip;        // k_wide_cluster: 1 when `next` holds the frontier
+  uint32_t pad;
 };
 
 struct P {
@@ -354,6 +360,408 @@ __global__ void __launch_bounds__(BLOCK_T) k_wide_round(const P p) {
   }
 }
 
+// ---- energies of one, two or four words: antichains in shared memory ----------
+// A candidate at a time against an antichain in global memory is a chain of a
+// few hundred cycles per candidate, with one lane busy while a list of one
+// energy is updated.  Here 32 candidates, taken across the successors' lists,
+// are updated by one lane each and inserted together: every lane compares its
+// candidate with all members (broadcast reads of shared memory), the ones left
+// meet one another by shuffles.  What remains, and its order, is what inserting
+// them in turn leaves: the members without a candidate below them, then the
+// candidates without a member at or below, a strictly smaller candidate or an
+// equal earlier one.  An antichain beyond SCAP members is left to k_wide_round
+// (Ctr::n_ovf).
+constexpr uint32_t SCAP = 256;
+template <int ES>
+struct SWarp {
+  uint32_t A[SCAP * ES], B[SCAP * ES];  // members
+  uint32_t Y[32 * ES];                  // a chunk of updated energies
+  uint32_t inc[32];
+  uint8_t fl[SCAP];                     // own energy (attacker tie rule)
+};
+
+template <int ES>
+__device__ __forceinline__ bool leq_es(const uint32_t (&a)[ES], const uint32_t (&b)[ES], const Swar &sw) {
+  bool r = true;
+#pragma unroll
+  for (int w = 0; w < ES; w++) r = r && leq_w(a[w], b[w], sw);
+  return r;
+}
+template <int ES>
+__device__ __forceinline__ bool eq_es(const uint32_t (&a)[ES], const uint32_t (&b)[ES]) {
+  bool r = true;
+#pragma unroll
+  for (int w = 0; w < ES; w++) r = r && a[w] == b[w];
+  return r;
+}
+
+// Insert the lanes' candidates (valid ones, in lane order) into the n members
+// at M.  false: no room.
+template <int ES>
+__device__ __forceinline__ bool insert32(const P &p, uint32_t *M, uint8_t *fl, uint32_t &n, const uint32_t (&x)[ES],
+                                         bool valid, bool own, uint32_t lane) {
+  constexpr uint32_t FULL = 0xffffffffu;
+  // Most candidates lie above a member: that is looked for first, four members
+  // at a time until every lane has one; only the candidates left are compared
+  // the other way, each with 32 members at once.
+  bool dom = !valid;
+  for (uint32_t m0 = 0; m0 < n && !__all_sync(FULL, dom); m0 += 4u) {
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; k++) {
+      const uint32_t m = min(m0 + k, n - 1u);
+      uint32_t mv[ES];
+#pragma unroll
+      for (int w = 0; w < ES; w++) mv[w] = M[m * ES + w];
+      if (leq_es<ES>(mv, x, p.sw)) {
+        dom = true;
+        if (own && valid && eq_es<ES>(mv, x)) fl[m] = 1;
+      }
+    }
+  }
+  bool live = !dom;
+  uint32_t lm = __ballot_sync(FULL, live);
+  for (uint32_t r = lm; r; r &= r - 1u) {
+    const uint32_t j = (uint32_t)__ffs((int)r) - 1u;
+    uint32_t xj[ES];
+#pragma unroll
+    for (int w = 0; w < ES; w++) xj[w] = __shfl_sync(FULL, x[w], j);
+    if (j != lane && leq_es<ES>(xj, x, p.sw) && (j < lane || !eq_es<ES>(xj, x))) live = false;
+  }
+  lm = __ballot_sync(FULL, live);
+  if (!lm) return true;
+  uint32_t rm = 0;  // bit k: member 32k + lane leaves
+  for (uint32_t r = lm; r; r &= r - 1u) {
+    const uint32_t j = (uint32_t)__ffs((int)r) - 1u;
+    uint32_t xj[ES];
+#pragma unroll
+    for (int w = 0; w < ES; w++) xj[w] = __shfl_sync(FULL, x[w], j);
+    for (uint32_t m = lane; m < n; m += 32u) {
+      uint32_t mv[ES];
+#pragma unroll
+      for (int w = 0; w < ES; w++) mv[w] = M[m * ES + w];
+      if (leq_es<ES>(xj, mv, p.sw)) rm |= 1u << (m >> 5);
+    }
+  }
+  const bool any_rm = __any_sync(FULL, rm != 0u);
+  __syncwarp();
+  if (any_rm) {
+    uint32_t out = 0;
+    for (uint32_t b0 = 0; b0 < n; b0 += 32u) {
+      const uint32_t m = b0 + lane;
+      const bool keep = m < n && !((rm >> (b0 >> 5)) & 1u);
+      uint32_t mv[ES];
+      uint8_t f = 0;
+      if (keep) {
+#pragma unroll
+        for (int w = 0; w < ES; w++) mv[w] = M[m * ES + w];
+        f = fl[m];
+      }
+      const uint32_t bal = __ballot_sync(FULL, keep);
+      __syncwarp();
+      if (keep) {
+        const uint32_t d = out + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+        for (int w = 0; w < ES; w++) M[d * ES + w] = mv[w];
+        fl[d] = f;
+      }
+      __syncwarp();
+      out += (uint32_t)__popc(bal);
+    }
+    n = out;
+  }
+  const uint32_t bal = __ballot_sync(FULL, live);
+  const uint32_t k = (uint32_t)__popc(bal);
+  if (n + k > SCAP) return false;
+  if (live) {
+    const uint32_t d = n + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+    for (int w = 0; w < ES; w++) M[d * ES + w] = x[w];
+    fl[d] = own ? 1 : 0;
+  }
+  n += k;
+  __syncwarp();
+  return true;
+}
+
+// solve_one with the antichains in shared memory.
+template <int ES>
+__device__ bool solve_es(const P &p, uint32_t slot, SWarp<ES> &s, uint32_t lane, unsigned long long &edges,
+                         unsigned long long &bytes) {
+  constexpr uint32_t FULL = 0xffffffffu;
+  const uint32_t v = p.front[slot];
+  const uint32_t e0 = p.row[v], e1 = p.row[v + 1], deg = e1 - e0;
+  const bool attacker = p.att[v] != 0;
+  const unsigned long long dv = p.desc[v];
+  constexpr unsigned long long esb = 4ull * ES;
+  uint32_t *A = s.A, *B = s.B;
+  uint32_t n = 0;
+  if (!attacker) {
+    // defenders wait until every successor has a list (energygame.rs:789-792)
+    bool empty = false;
+    for (uint32_t k = e0 + lane; k < e1; k += 32) empty |= dcnt(p.desc[p.col[k]]) == 0;
+    if (deg == 0 || __any_sync(FULL, empty)) {
+      if (lane == 0) p.slot_new[slot] = NOCHANGE;
+      return true;
+    }
+  }
+  unsigned long long by = 12ull + 16ull * deg;
+  auto fetch = [&](unsigned long long d, uint32_t q, const uint32_t *u, uint32_t (&x)[ES]) {
+    const uint32_t *src = p.arena + (doff(d) + q) * ES;
+#pragma unroll
+    for (int w = 0; w < ES; w++) x[w] = src[w];
+    wide_inv_update(p.wc, x, u);
+  };
+  if (attacker) {
+    for (uint32_t k0 = e0; k0 < e1; k0 += 32u) {
+      const uint32_t k = k0 + lane;
+      const unsigned long long d = k < e1 ? p.desc[p.col[k]] : 0ull;
+      const uint32_t c = k < e1 ? dcnt(d) : 0u;
+      uint32_t inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, inc, o);
+        if (lane >= (uint32_t)o) inc += y;
+      }
+      const uint32_t total = __shfl_sync(FULL, inc, 31);
+      by += esb * total;
+      __syncwarp();
+      s.inc[lane] = inc;
+      __syncwarp();
+      for (uint32_t t0 = 0; t0 < total; t0 += 32u) {
+        const uint32_t t = t0 + lane;
+        const bool valid = t < total;
+        uint32_t lo = 0;  // the successor whose range holds candidate t
+        if (valid) {
+          uint32_t hi = 31;
+          while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (s.inc[mid] > t) hi = mid;
+            else lo = mid + 1;
+          }
+        }
+        const unsigned long long dk = __shfl_sync(FULL, d, lo);
+        uint32_t x[ES] = {};
+        if (valid) fetch(dk, t - (lo ? s.inc[lo - 1] : 0u), p.wt + (unsigned long long)(k0 + lo) * p.us, x);
+        if (!insert32<ES>(p, A, s.fl, n, x, valid, false, lane)) return false;
+      }
+    }
+    by += esb * dcnt(dv);
+    for (uint32_t q0 = 0; q0 < dcnt(dv); q0 += 32u) {
+      const bool valid = q0 + lane < dcnt(dv);
+      uint32_t x[ES] = {};
+      if (valid) fetch(dv, q0 + lane, nullptr, x);
+      if (!insert32<ES>(p, A, s.fl, n, x, valid, true, lane)) return false;
+    }
+    edges += deg;
+    // changed iff a kept energy came from a successor (attack_minimize.wgsl:95-101)
+    bool from_succ = false;
+    for (uint32_t j = lane; j < n; j += 32) from_succ |= s.fl[j] == 0;
+    if (!__any_sync(FULL, from_succ)) {
+      if (lane == 0) p.slot_new[slot] = NOCHANGE;
+      bytes += by;
+      return true;
+    }
+  } else {
+    for (uint32_t k = e0; k < e1; k++) {
+      const unsigned long long d = p.desc[p.col[k]];
+      const uint32_t *u = p.wt + (unsigned long long)k * p.us;
+      by += esb * dcnt(d);
+      uint32_t nb = 0;
+      for (uint32_t q0 = 0; q0 < dcnt(d); q0 += 32u) {
+        const uint32_t ny = min(32u, dcnt(d) - q0);
+        uint32_t x[ES] = {};
+        if (lane < ny) fetch(d, q0 + lane, u, x);
+        if (k == e0) {
+          // a single successor's updated list as is, else the first list minimised
+          if (deg == 1u) {
+            if (n + ny > SCAP) return false;
+            if (lane < ny) {
+#pragma unroll
+              for (int w = 0; w < ES; w++) A[(n + lane) * ES + w] = x[w];
+            }
+            n += ny;
+            __syncwarp();
+          } else if (!insert32<ES>(p, A, s.fl, n, x, lane < ny, false, lane)) {
+            return false;
+          }
+          continue;
+        }
+        // minimal elements of the pairwise suprema, in the order (energy, member)
+        if (lane < ny) {
+#pragma unroll
+          for (int w = 0; w < ES; w++) s.Y[lane * ES + w] = x[w];
+        }
+        __syncwarp();
+        for (uint32_t i0 = 0; i0 < ny * n; i0 += 32u) {
+          const uint32_t i = i0 + lane;
+          const bool valid = i < ny * n;
+          uint32_t z[ES] = {};
+          if (valid) {
+            const uint32_t yq = i / n, am = i - yq * n;
+#pragma unroll
+            for (int w = 0; w < ES; w++) z[w] = max_w(A[am * ES + w], s.Y[yq * ES + w], p.sw);
+          }
+          if (!insert32<ES>(p, B, s.fl, nb, z, valid, false, lane)) return false;
+        }
+        __syncwarp();
+      }
+      if (k != e0) {
+        uint32_t *t = A;
+        A = B;
+        B = t;
+        n = nb;
+      }
+    }
+    edges += deg;
+    // changed iff the list differs from the old one (EnergyArray ==,
+    // energy.rs:334-350: same length and every new energy in the old list)
+    bool same = dcnt(dv) == n;
+    if (same) {
+      bool miss = false;
+      for (uint32_t j = lane; j < n; j += 32) {
+        bool found = false;
+        for (uint32_t q = 0; q < n && !found; q++) {
+          const uint32_t *o = p.arena + (doff(dv) + q) * ES;
+          bool eq = true;
+#pragma unroll
+          for (int w = 0; w < ES; w++) eq = eq && o[w] == A[j * ES + w];
+          found = eq;
+        }
+        miss |= !found;
+      }
+      same = !__any_sync(FULL, miss);
+    }
+    if (same) {
+      if (lane == 0) p.slot_new[slot] = NOCHANGE;
+      bytes += by;
+      return true;
+    }
+  }
+  unsigned long long off = 0;
+  if (lane == 0) off = atomicAdd(&p.ctr->arena_top, (unsigned long long)n);
+  off = __shfl_sync(FULL, off, 0);
+  bytes += by;
+  if (off + n > p.arena_cap) {
+    if (lane == 0) {
+      atomicExch(&p.ctr->arena_full, 1u);
+      p.slot_new[slot] = NOCHANGE;
+    }
+    return true;
+  }
+  for (uint32_t w = lane; w < n * ES; w += 32) p.arena[off * ES + w] = A[w];
+  bytes += esb * n;
+  if (lane == 0) p.slot_new[slot] = (off << CNT_BITS) | n;
+  __syncwarp();
+  return true;
+}
+
+// A round by all warps of the device (the first attempt at every slot).
+template <int ES>
+__global__ void __launch_bounds__(BLOCK_T) k_wide_round_es(const P p) {
+  __shared__ SWarp<ES> sw[WARPS];
+  const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+  unsigned long long edges = 0, bytes = 0, pos = 0;
+  for (;;) {
+    uint32_t i = 0;
+    if (lane == 0) i = atomicAdd(&p.ctr->next_slot, 1u);
+    i = __shfl_sync(0xffffffffu, i, 0);
+    if (i >= p.n_items) break;
+    if (!solve_es<ES>(p, i, sw[wib], lane, edges, bytes)) {
+      if (lane == 0) p.ovf[atomicAdd(&p.ctr->n_ovf, 1u)] = i;
+    } else {
+      pos++;
+    }
+    __syncwarp();
+  }
+  if (lane == 0 && pos) {
+    atomicAdd(&p.ctr->positions, pos);
+    atomicAdd(&p.ctr->edges, edges);
+    atomicAdd(&p.ctr->bytes, bytes);
+  }
+}
+
+// Rounds inside one launch of a cluster of blocks, for games of some ten
+// thousand positions: three barriers a round in place of three launches, four
+// fills, two read-backs and the waits for them.  Leaves before the commit of a
+// round that met a full arena or antichains beyond SCAP members, for the host
+// to finish that round.
+constexpr uint32_t CWARPS = 16, CTHREADS = 32 * CWARPS;
+template <int ES>
+__global__ void __launch_bounds__(CTHREADS, 1) k_wide_cluster(P p, uint32_t fs, uint32_t max_rounds) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const uint32_t rank = cl.block_rank(), blocks = cl.num_blocks();
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  SWarp<ES> &s = ((SWarp<ES> *)dsm)[warp];
+  const uint32_t gw = warp * blocks + rank, warps = blocks * CWARPS;
+  const uint32_t tid = gw * 32u + lane, threads = warps * 32u;
+  Ctr *c = p.ctr;
+  unsigned long long edges = 0, bytes = 0, pos = 0;
+  uint32_t *front = const_cast<uint32_t *>(p.front), *next = p.next;
+  uint32_t rounds = 0, flip = 0;
+  bool stop = false;
+  while (fs && rounds < max_rounds) {
+    p.front = front;
+    // the fuller warps of a round are not known beforehand: slots by a counter
+    for (;;) {
+      uint32_t i = 0;
+      if (lane == 0) i = atomicAdd(&c->next_slot, 1u);
+      i = __shfl_sync(0xffffffffu, i, 0);
+      if (i >= fs) break;
+      if (!solve_es<ES>(p, i, s, lane, edges, bytes)) {
+        if (lane == 0) p.ovf[atomicAdd(&c->n_ovf, 1u)] = i;
+      } else {
+        pos++;
+      }
+      __syncwarp();
+    }
+    cl.sync();
+    stop = *(volatile uint32_t *)&c->n_ovf != 0u || *(volatile uint32_t *)&c->arena_full != 0u;
+    if (stop) break;
+    for (uint32_t k = tid; k < fs; k += threads) {
+      const unsigned long long d = p.slot_new[k];
+      if (d == NOCHANGE) continue;
+      const uint32_t v = front[k];
+      p.desc[v] = d;
+      for (uint32_t e = p.rrow[v]; e < p.rrow[v + 1]; e++) {
+        const uint32_t u = p.rcol[e];
+        atomicOr(&p.mark[u >> 5], 1u << (u & 31u));
+      }
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+      c->next_slot = 0u;
+      c->next_size = 0u;
+    }
+    cl.sync();
+    for (uint32_t w = tid; w < p.mwords; w += threads) {
+      uint32_t b = p.mark[w];
+      if (!b) continue;
+      p.mark[w] = 0u;
+      uint32_t at = atomicAdd(&c->next_size, (uint32_t)__popc(b));
+      for (; b; b &= b - 1u) next[at++] = w * 32u + (uint32_t)__ffs((int)b) - 1u;
+    }
+    cl.sync();
+    fs = *(volatile uint32_t *)&c->next_size;
+    uint32_t *t = front;
+    front = next;
+    next = t;
+    flip ^= 1u;
+    rounds++;
+    cl.sync();  // everyone has read the size
+  }
+  if (lane == 0 && pos) {
+    atomicAdd(&c->positions, pos);
+    atomicAdd(&c->edges, edges);
+    atomicAdd(&c->bytes, bytes);
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    c->rounds = c->rounds + rounds;
+    c->next_size = fs;
+    c->flip = flip;
+  }
+  cl.sync();
+}
+
 // publish the round's lists and mark the predecessors of changed positions
 __global__ void k_wide_commit(const P p, uint32_t n_slots) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -417,35 +825,92 @@ __global__ void k_wide_redesc(unsigned long long *desc, const unsigned long long
                                        "%s: %s", #x, cudaGetErrorString(e_));           \
   } while (0)
 
-// device buffers of one solve, released with the stream
+// Device buffers of one solve from the engine's pool (all work is on the
+// engine's stream).  The device's stream-ordered pool gives its memory back at
+// every wait unless told otherwise: a solve's 18 buffers then cost 10 to 60 ms.
 struct Bufs {
-  cudaStream_t S;
-  std::vector<void *> ptrs;
+  Engine &eng;
+  std::vector<std::pair<void *, size_t>> ptrs;
   template <class T>
   geq_status get(T *&p, size_t n) {
-    void *q = nullptr;
-    const cudaError_t e = cudaMallocAsync(&q, std::max<size_t>(n, 1) * sizeof(T), S);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail(GEQ_ERR_OUT_OF_MEMORY, "device allocation of %zu bytes for the wide solver failed",
-                  std::max<size_t>(n, 1) * sizeof(T));
-    }
-    ptrs.push_back(q);
+    const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+    void *q = eng.pool_get(bytes);
+    if (!q) return fail(GEQ_ERR_OUT_OF_MEMORY, "device allocation of %zu bytes for the wide solver failed", bytes);
+    ptrs.emplace_back(q, bytes);
     p = (T *)q;
     return GEQ_OK;
   }
   void put(void *q) {
     for (auto &x : ptrs)
-      if (x == q) {
-        cudaFreeAsync(q, S);
-        x = nullptr;
+      if (x.first == q) {
+        eng.pool_put(q, x.second);
+        x.first = nullptr;
       }
   }
   ~Bufs() {
-    for (void *q : ptrs)
-      if (q) cudaFreeAsync(q, S);
+    cudaStreamSynchronize((cudaStream_t)eng.stream_handle());  // error paths leave work behind
+    for (auto &x : ptrs)
+      if (x.first) eng.pool_put(x.first, x.second);
   }
 };
+
+// The cluster kernels on the current device (once): blocks per cluster, 0: none.
+template <int ES>
+static uint32_t cluster_setup_es() {
+  const size_t smem = sizeof(SWarp<ES>) * CWARPS;
+  if (cudaFuncSetAttribute(k_wide_cluster<ES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_wide_cluster<ES>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  for (uint32_t b = 16; b >= 8; b /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(b);
+    cfg.blockDim = dim3(CTHREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = b;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_wide_cluster<ES>, &cfg) == cudaSuccess && n > 0) return b;
+    cudaGetLastError();
+  }
+  return 0;
+}
+static uint32_t cluster_blocks(int device, uint32_t es) {
+  static std::once_flag once[64];
+  static uint32_t blocks[64] = {};
+  if (device < 0 || device >= 64 || (es != 1 && es != 2 && es != 4)) return 0;
+  std::call_once(once[device], [device]() {
+    blocks[device] = std::min({cluster_setup_es<1>(), cluster_setup_es<2>(), cluster_setup_es<4>()});
+  });
+  return blocks[device];
+}
+template <int ES>
+static cudaError_t launch_cluster_es(const P &p, uint32_t blocks, uint32_t fs, uint32_t max_rounds, cudaStream_t S) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(CTHREADS);
+  cfg.dynamicSmemBytes = sizeof(SWarp<ES>) * CWARPS;
+  cfg.stream = S;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = blocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_wide_cluster<ES>, p, fs, max_rounds);
+}
+// Games of up to so many positions run their rounds inside cluster launches.
+// Median per call on one B200, one warp per position in global scratch / these kernels without and
+// with the cluster, 8, 16 and 24 warps a block: conf {30, 3}, 12,000 positions
+// 21.2 / 10.0 / 8.6, 8.1, 8.6 ms; 300 positions 1.42 / 1.11 / 0.49, 0.50, 0.51
+// ms; {16, 7}, 20,000 positions 6.1 / 5.2 / 5.0, 4.2, 4.2 ms.
+constexpr uint32_t WIDE_CLUSTER_POSITIONS = 65536;
+constexpr uint32_t WIDE_CLUSTER_ROUNDS = 256;       // per launch
 
 static geq_status check_game(const GameInput &gi, const Conf &c) {
   const geq_game_graph &g = gi.g;
@@ -461,6 +926,9 @@ static geq_status check_game(const GameInput &gi, const Conf &c) {
   const uint64_t fields_bits = (uint64_t)ub * c.elements;
   for (uint64_t k = 0; k < m; k++) {
     const uint32_t *u = g.weights + k * us;
+    uint32_t any = 0;
+    for (uint32_t w = 0; w < us; w++) any |= u[w];
+    if (!any) continue;
     for (uint32_t i = 0; i < c.elements; i++) {
       const uint32_t bit = i * ub, code = (u[bit >> 5] >> (bit & 31u)) & um;
       if (code >= 2 && code - 2 >= c.elements)
@@ -475,8 +943,10 @@ static geq_status check_game(const GameInput &gi, const Conf &c) {
 }
 
 // One game on the engine's stream.
-static geq_status solve_one_game(cudaStream_t S, int n_sms, const GameInput &gi, const Conf &c, geq_solution &sol,
+static geq_status solve_one_game(Engine &eng, int device, const GameInput &gi, const Conf &c, geq_solution &sol,
                                  uint32_t g_index) {
+  cudaStream_t S = (cudaStream_t)eng.stream_handle();
+  const int n_sms = eng.n_sms;
   const geq_game_graph &g = gi.g;
   const uint32_t n = g.n_vertices, es = c.energy_size(), us = c.update_size();
   const uint64_t m = g.row_offsets[n];
@@ -510,7 +980,7 @@ static geq_status solve_one_game(cudaStream_t S, int n_sms, const GameInput &gi,
   }
   const unsigned long long init_e = init_words.size() / es;
 
-  Bufs B{S, {}};
+  Bufs B{eng, {}};
   P p{};
   uint32_t *d_row, *d_col, *d_wt, *d_rrow, *d_rcol, *d_front, *d_next, *d_ovf, *d_mark, *d_reach, *d_arena,
       *d_scratch;
@@ -529,7 +999,10 @@ static geq_status solve_one_game(cudaStream_t S, int n_sms, const GameInput &gi,
   const uint32_t max_warps = (uint32_t)n_sms * 16;
   unsigned long long scratch_words = 1ull << 14;  // per warp
   uint32_t scratch_warps = max_warps;
-  if ((st = B.get(d_scratch, scratch_words * scratch_warps))) return st;
+  // the scratch of energies of one, two or four words is taken when an
+  // antichain outgrows shared memory
+  d_scratch = nullptr;
+  if (es != 1 && es != 2 && es != 4 && (st = B.get(d_scratch, scratch_words * scratch_warps))) return st;
 
   WCU(cudaMemcpyAsync(d_row, g.row_offsets, (n + 1) * 4ull, cudaMemcpyHostToDevice, S));
   if (m) {
@@ -597,25 +1070,56 @@ static geq_status solve_one_game(cudaStream_t S, int n_sms, const GameInput &gi,
   p.front = d_front;
   p.next = d_next;
   uint64_t rounds = 0;
+  const uint32_t cluster = n <= WIDE_CLUSTER_POSITIONS ? cluster_blocks(device, es) : 0u;
   const auto t_start = std::chrono::steady_clock::now();
   while (fsize) {
+    bool first_try = true;  // of this round's slots
+    if (cluster) {
+      // rounds in one launch; a round it left unfinished goes on below
+      WCU(cudaMemsetAsync(&d_ctr->next_slot, 0, 12, S));  // next_slot, n_ovf, arena_full
+      p.slots = nullptr;
+      WCU(es == 1   ? launch_cluster_es<1>(p, cluster, fsize, WIDE_CLUSTER_ROUNDS, S)
+          : es == 2 ? launch_cluster_es<2>(p, cluster, fsize, WIDE_CLUSTER_ROUNDS, S)
+                    : launch_cluster_es<4>(p, cluster, fsize, WIDE_CLUSTER_ROUNDS, S));
+      launches++;
+      WCU(cudaMemcpyAsync(&h, d_ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, S));
+      WCU(cudaStreamSynchronize(S));
+      fsize = h.next_size;
+      if (h.flip) std::swap(d_front, d_next);
+      p.front = d_front;
+      p.next = d_next;
+      if (std::chrono::steady_clock::now() - t_start > std::chrono::seconds(600))
+        return fail(GEQ_ERR_TIMEOUT, "no fixpoint after 600 s (%llu rounds)", (unsigned long long)(rounds + h.rounds));
+      if (!h.n_ovf && !h.arena_full) continue;
+      first_try = false;
+    }
     rounds++;
     if (std::chrono::steady_clock::now() - t_start > std::chrono::seconds(600))
       return fail(GEQ_ERR_TIMEOUT, "no fixpoint after 600 s (%llu rounds)", (unsigned long long)rounds);
     // the round, repeated for positions whose antichain outgrew the scratch
     p.slots = nullptr;
     p.n_items = fsize;
+    const bool shared_ac = es == 1 || es == 2 || es == 4;
+    bool fresh = shared_ac;  // all slots, antichains in shared memory; else in the warps' scratch
     for (;;) {
-      WCU(cudaMemsetAsync(&d_ctr->next_slot, 0, 4, S));
-      WCU(cudaMemsetAsync(&d_ctr->n_ovf, 0, 4, S));
-      WCU(cudaMemsetAsync(&d_ctr->arena_full, 0, 4, S));
-      const uint32_t warps = std::min<uint32_t>(scratch_warps, std::max<uint32_t>(p.n_items, 1));
-      p.n_warps = warps;
-      k_wide_round<<<(warps + WARPS - 1) / WARPS, BLOCK_T, smem, S>>>(p);
-      launches++;
-      WCU(cudaGetLastError());
-      WCU(cudaMemcpyAsync(&h, d_ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, S));
-      WCU(cudaStreamSynchronize(S));
+      if (first_try || !cluster) {
+        WCU(cudaMemsetAsync(&d_ctr->next_slot, 0, 12, S));  // next_slot, n_ovf, arena_full
+        const uint32_t warps = std::min<uint32_t>(scratch_warps, std::max<uint32_t>(p.n_items, 1));
+        p.n_warps = warps;
+        if (fresh) {
+          const unsigned blocks = std::min<unsigned>((p.n_items + WARPS - 1) / WARPS, (unsigned)n_sms * 4u);
+          if (es == 1) k_wide_round_es<1><<<blocks, BLOCK_T, 0, S>>>(p);
+          else if (es == 2) k_wide_round_es<2><<<blocks, BLOCK_T, 0, S>>>(p);
+          else k_wide_round_es<4><<<blocks, BLOCK_T, 0, S>>>(p);
+        } else {
+          k_wide_round<<<(warps + WARPS - 1) / WARPS, BLOCK_T, smem, S>>>(p);
+        }
+        launches++;
+        WCU(cudaGetLastError());
+        WCU(cudaMemcpyAsync(&h, d_ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, S));
+        WCU(cudaStreamSynchronize(S));
+      }
+      first_try = true;
       if (h.arena_full) {
         // compact the committed lists into a larger arena and run the round again
         std::vector<unsigned long long> hd(n), noff(n);
@@ -643,14 +1147,16 @@ static geq_status solve_one_game(cudaStream_t S, int n_sms, const GameInput &gi,
         WCU(cudaMemcpyAsync(&d_ctr->arena_top, &live, 8, cudaMemcpyHostToDevice, S));
         p.slots = nullptr;
         p.n_items = fsize;
+        fresh = shared_ac;
         continue;
       }
       if (!h.n_ovf) break;
-      // positions whose antichain did not fit: again with 8x the scratch
-      // each, on as many warps as the memory allows
-      scratch_words *= 8;
+      // positions whose antichain did not fit: in the warps' scratch, then
+      // again with 8x the scratch each, on as many warps as the memory allows
+      if (!fresh) scratch_words *= 8;
+      fresh = false;
       if (scratch_words > (1ull << 31)) return fail(GEQ_ERR_OUT_OF_MEMORY, "antichain beyond 8 GB of warp scratch");
-      B.put(d_scratch);
+      if (d_scratch) B.put(d_scratch);
       scratch_warps = (uint32_t)std::max<unsigned long long>(
           1, std::min<unsigned long long>(max_warps, (4ull << 30) / (scratch_words * 4)));
       if ((st = B.get(d_scratch, scratch_words * scratch_warps))) return st;
@@ -702,7 +1208,7 @@ static geq_status solve_one_game(cudaStream_t S, int n_sms, const GameInput &gi,
   WCU(cudaStreamSynchronize(S));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ev0, ev1);
-  sol.stats.rounds += rounds;
+  sol.stats.rounds += rounds + h.rounds;
   sol.stats.positions_computed += h.positions;
   sol.stats.edges_relaxed += h.edges;
   sol.stats.algorithmic_bytes += h.bytes;
@@ -738,7 +1244,6 @@ geq_status solve_wide(Engine &e, int device, std::vector<GameInput> &in, geq_sol
     int prev, dev;
     ~Restore() { if (prev != dev && prev >= 0) cudaSetDevice(prev); }
   } restore{prev, device};
-  cudaStream_t S = (cudaStream_t)e.stream_handle();
   sol.energy_size = c.energy_size();
   for (uint32_t g = 0; g < in.size(); g++) {
     GameInput &gi = in[g];
@@ -748,7 +1253,7 @@ geq_status solve_wide(Engine &e, int device, std::vector<GameInput> &in, geq_sol
       gi.n_reach = (uint32_t)gi.reach_storage.size();
       gi.std_reach = false;
     }
-    const geq_status st = wide::solve_one_game(S, e.n_sms, gi, c, sol, g);
+    const geq_status st = wide::solve_one_game(e, device, gi, c, sol, g);
     if (st) return st;
   }
   return GEQ_OK;

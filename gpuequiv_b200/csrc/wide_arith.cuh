@@ -60,24 +60,70 @@ __host__ __device__ __forceinline__ uint32_t swar_max(uint32_t a, uint32_t b, co
   return ((be & me) | (ae & ~me)) | (((bo & mo) | (ao & ~mo)) << s.k);
 }
 
+// field-wise min
+__host__ __device__ __forceinline__ uint32_t swar_min(uint32_t a, uint32_t b, const Swar &s) {
+  if (s.k == 32u) return a < b ? a : b;
+  return a ^ b ^ swar_max(a, b, s);
+}
+
 // Inverse update of one energy in place (UPDATE1 then UPDATE_MIN,
 // shadergen.rs:103-128, as inv_update in attack_update.wgsl:45-61): every
 // field +1 in u32 arithmetic where the code is 1 (Decrement), then min with
 // max; then, in index order, a field with code k+2 (Min into k) raises field
 // k to its value.  u = the update words, null for the zero update (the
-// clamp alone, applied to an attacker's own energies).
-__host__ __device__ inline void wide_inv_update(const WideConf &c, uint32_t *x, const uint32_t *u) {
-  for (uint32_t i = 0; i < c.el; i++) {
-    const uint32_t code = u ? getf(u, i, c.ub, c.um) : 0u;
-    const uint32_t f = getf(x, i, c.eb, c.em) + (code == 1u ? 1u : 0u);
-    setf(x, i, c.eb, c.em, f < c.mx ? f : c.mx);
+// clamp alone, applied to an attacker's own energies).  Few fields of an update
+// have a code, so the clamp goes word by word and the codes' words are
+// searched for the set ones (field by field it was two loops over up to 30
+// fields per energy).
+__host__ __device__ __forceinline__ uint32_t low_bit(uint32_t x) {
+#ifdef __CUDA_ARCH__
+  return (uint32_t)__ffs((int)x) - 1u;
+#else
+  return (uint32_t)__builtin_ctz(x);
+#endif
+}
+__host__ __device__ __forceinline__ void wide_inv_update(const WideConf &c, uint32_t *x, const uint32_t *u) {
+  const uint32_t fpw = 32u / c.eb, es = (c.el + fpw - 1u) / fpw;
+  const uint32_t upw = 32u / c.ub, us = u ? (c.el + upw - 1u) / upw : 0u;
+  bool merges = false, decs = false;
+  for (uint32_t w = 0; w < us; w++) {
+    uint32_t rest = u[w];
+    while (rest) {
+      const uint32_t f = low_bit(rest) / c.ub, code = (rest >> (f * c.ub)) & c.um;
+      rest &= ~(c.um << (f * c.ub));
+      merges |= code >= 2u;
+      decs |= code == 1u;
+    }
   }
-  if (!u) return;
-  for (uint32_t i = 0; i < c.el; i++) {
-    const uint32_t code = getf(u, i, c.ub, c.um);
-    if (code >= 2u && code - 2u < c.el) {
-      const uint32_t t = code - 2u, a = getf(x, t, c.eb, c.em), b = getf(x, i, c.eb, c.em);
-      if (b > a) setf(x, t, c.eb, c.em, b);
+  // the decremented fields from their unclamped values
+  if (decs)
+    for (uint32_t w = 0; w < us; w++) {
+      uint32_t rest = u[w];
+      while (rest) {
+        const uint32_t f = low_bit(rest) / c.ub, code = (rest >> (f * c.ub)) & c.um, i = w * upw + f;
+        rest &= ~(c.um << (f * c.ub));
+        if (code == 1u && i < c.el) {
+          const uint32_t v = getf(x, i, c.eb, c.em) + 1u;
+          setf(x, i, c.eb, c.em, v < c.mx ? v : c.mx);
+        }
+      }
+    }
+  if (c.mx != c.em) {
+    uint32_t all = 0;
+    for (uint32_t k = 0; k < fpw; k++) all |= c.mx << (k * c.eb);
+    const Swar sw = make_swar(c.eb);
+    for (uint32_t w = 0; w < es; w++) x[w] = swar_min(x[w], all, sw);
+  }
+  if (!merges) return;
+  for (uint32_t w = 0; w < us; w++) {
+    uint32_t rest = u[w];
+    while (rest) {
+      const uint32_t f = low_bit(rest) / c.ub, code = (rest >> (f * c.ub)) & c.um, i = w * upw + f;
+      rest &= ~(c.um << (f * c.ub));
+      if (code >= 2u && code - 2u < c.el && i < c.el) {
+        const uint32_t t = code - 2u, a = getf(x, t, c.eb, c.em), b = getf(x, i, c.eb, c.em);
+        if (b > a) setf(x, t, c.eb, c.em, b);
+      }
     }
   }
 }

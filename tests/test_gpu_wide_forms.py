@@ -1,0 +1,121 @@
+"""The forms of the multi-word solver's rounds against the oracle: antichains
+in shared memory (energies of one, two and four words) up to, at and beyond
+their 256 members, other energy sizes in the warps' scratch, games whose rounds
+run inside one launch (up to 65,536 positions) and larger ones."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from helpers import canon
+from oracle import ora
+
+pytestmark = pytest.mark.gpu
+
+CONFS = [(2, 65535), (3, 1000), (30, 3), (50, 3), (1, 0xFFFFFFFF), (5, 0xFFFFFFFF)]
+
+
+@pytest.fixture(scope="module")
+def geq():
+    import gpuequiv_b200 as geq
+    return geq
+
+
+@pytest.fixture(scope="module")
+def ctx(geq):
+    c = geq.Context(0)
+    yield c
+    c.close()
+
+
+def pack(geq, conf, values):
+    c = geq.EnergyConf(*conf)
+    out = np.zeros((len(values), c.energy_size()), np.uint32)
+    per = 32 // c.energy_bits()
+    for i in range(conf[0]):
+        shift = np.uint32(c.energy_bits() * (i % per))
+        out[:, i // per] |= values[:, i].astype(np.uint32) << shift
+    return out
+
+
+def update_words(geq, conf, codes):
+    c = geq.EnergyConf(*conf)
+    out = np.zeros((len(codes), c.update_size()), np.uint32)
+    per = 32 // c.update_bits()
+    for i in range(conf[0]):
+        out[:, i // per] |= codes[:, i].astype(np.uint32) << np.uint32(c.update_bits() * (i % per))
+    return out
+
+
+def run_both(geq, ctx, conf, row, col, wt, att, reach, offs, data):
+    from gpuequiv_b200._lib import check, geq_energy_lists, lib
+    cf = geq.EnergyConf(*conf)
+    es = cf.energy_size()
+    g = geq.GameGraph.from_csr(row, col, wt, att, cf)
+    view = g.c_view()
+    flat = np.ascontiguousarray(data.reshape(-1)) if data.size else np.zeros(1, np.uint32)
+    init = geq_energy_lists(len(att), es, offs.ctypes.data_as(C.POINTER(C.c_uint64)),
+                            flat.ctypes.data_as(C.POINTER(C.c_uint32)))
+    sol, out = C.c_void_p(), geq_energy_lists()
+    check(lib.geq_energy_game_run(ctx.h, C.byref(view), C.byref(init), reach.ctypes.data_as(C.POINTER(C.c_uint32)),
+                                  len(reach), C.byref(sol)))
+    check(lib.geq_solution_lists(sol, 0, C.byref(out)))
+    o = np.ctypeslib.as_array(out.offsets, shape=(len(att) + 1,)).astype(np.int64)
+    d = (np.ctypeslib.as_array(out.data, shape=(int(o[-1]) * es,)).copy() if o[-1] else
+         np.zeros(0, np.uint32)).reshape(-1, es)
+    lib.geq_solution_free(sol)
+    exp = ora.run_game(conf[0], conf[1], row, col, np.asarray(wt).reshape(-1), att, reach, init=(offs, flat)).lists()
+    assert np.array_equal(np.diff(o), [len(x) for x in exp])
+    for v in range(len(att)):
+        assert canon(d[o[v]:o[v + 1]]) == canon(exp[v]), f"position {v}"
+
+
+@pytest.mark.parametrize("conf", CONFS)
+@pytest.mark.parametrize("members", [1, 31, 32, 33, 255, 256, 257, 300])
+def test_antichain_sizes(geq, ctx, conf, members):
+    """0 (attacker) -> 1 (defender) -> 2 and 3 (attackers with given lists of
+    `members` energies); 4 (defender, one successor) -> 2; 0 -> 4."""
+    rng = np.random.default_rng(members)
+    el, mx = conf
+    lists = []
+    for _ in range(2):
+        v = rng.integers(0, min(mx, 3) + 1, (members, el)).astype(np.uint64)
+        if el > 1 and mx >= 300:  # an antichain: one element up, another down
+            v[:, 0] = np.arange(members)
+            v[:, 1] = members - np.arange(members)
+        lists.append(pack(geq, conf, v))
+    if members >= 255:  # keep the product of the two lists small
+        lists[1] = lists[1][:2]
+    row = np.array([0, 2, 4, 4, 4, 5], np.uint32)
+    col = np.array([1, 4, 2, 3, 2], np.uint32)
+    codes = np.zeros((5, el), np.uint32)
+    codes[0, 0] = 1
+    codes[2, el - 1] = 1
+    if el > 2:
+        codes[3, 1] = 2 + 2
+        codes[4, 2] = 1
+    offs = np.array([0, 0, 0, len(lists[0]), len(lists[0]) + len(lists[1]), len(lists[0]) + len(lists[1])], np.uint64)
+    run_both(geq, ctx, conf, row, col, update_words(geq, conf, codes), np.array([1, 0, 1, 1, 0], np.uint8),
+             np.array([2, 3], np.uint32), offs, np.concatenate(lists))
+
+
+@pytest.mark.parametrize("conf", [(30, 3), (1, 0xFFFFFFFF)])
+@pytest.mark.parametrize("n", [1, 33, 65536, 65537])
+def test_game_sizes(geq, ctx, conf, n):
+    rng = np.random.default_rng(n)
+    att = (rng.random(n) < 0.6).astype(np.uint8)
+    deg = rng.integers(0, 3, n)
+    row = np.zeros(n + 1, np.uint32)
+    row[1:] = np.cumsum(deg)
+    m = int(row[-1])
+    col = rng.integers(0, n, m).astype(np.uint32)
+    codes = np.zeros((m, conf[0]), np.uint32)
+    codes[np.arange(m), rng.integers(0, conf[0], m)] = rng.random(m) < 0.2
+    reach = np.nonzero((att == 0) & (deg == 0))[0].astype(np.uint32)
+    offs = np.zeros(n + 1, np.uint64)
+    offs[1:] = np.cumsum((att == 0) & (deg == 0))
+    es = geq.EnergyConf(*conf).energy_size()
+    run_both(geq, ctx, conf, row, col, update_words(geq, conf, codes), att, reach, offs,
+             np.zeros((int(offs[-1]), es), np.uint32))
