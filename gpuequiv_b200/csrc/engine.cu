@@ -2342,18 +2342,43 @@ __global__ void k_arena_counts(const unsigned long long *desc, unsigned long lon
   }
 }
 
-__global__ void k_gather(const unsigned long long *desc, unsigned long long n, const unsigned long long *goff,
-                         const uint32_t *arena, uint32_t ib, uint32_t ibm, uint32_t *out) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const unsigned long long gw = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
-  const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-  for (unsigned long long v = gw; v < n; v += nw) {
-    const unsigned long long d = desc[v];
-    const uint32_t c = dcnt(d);
-    const unsigned long long go = goff[v];
-    for (uint32_t q = lane; q < c; q += 32u)
-      out[go + q] = dinl(d) ? ((uint32_t)(d >> (q * ib)) & ibm) : arena[doff(d) + q];
+// Energies of positions of a tile side by side: most lists are one to five
+// energies inside a descriptor, so a thread takes a position and the tile's
+// words go out together (a warp per position, with one lane in ten busy,
+// took 0.85 ms for 7.6M positions on one B200; this form 0.066 ms).  `at(v)` is
+// the position of item v, goff its exclusive offsets (n + 1).
+constexpr uint32_t GATHER_T = 256, GATHER_WORDS = 2048;
+template <class At>
+__device__ __forceinline__ void gather_tiles(const unsigned long long *desc, unsigned long long n, const At &at,
+                                             const unsigned long long *goff, const uint32_t *arena, uint32_t ib,
+                                             uint32_t ibm, uint32_t *out) {
+  __shared__ uint32_t w[GATHER_WORDS];
+  for (unsigned long long t0 = (unsigned long long)blockIdx.x * GATHER_T; t0 < n;
+       t0 += (unsigned long long)gridDim.x * GATHER_T) {
+    const unsigned long long v = t0 + threadIdx.x, te = min(n, t0 + GATHER_T);
+    const unsigned long long o0 = goff[t0], words = goff[te] - o0;
+    const bool staged = words <= GATHER_WORDS;
+    if (v < te) {
+      const unsigned long long d = desc[at(v)], o = goff[v] - o0;
+      const uint32_t c = dcnt(d);
+      uint32_t *to = staged ? w + o : out + o0 + o;
+      if (dinl(d)) {
+        for (uint32_t q = 0; q < c; q++) to[q] = (uint32_t)(d >> (q * ib)) & ibm;
+      } else {
+        const uint32_t *src = arena + doff(d);
+        for (uint32_t q = 0; q < c; q++) to[q] = src[q];
+      }
+    }
+    __syncthreads();
+    if (staged)
+      for (uint32_t i = threadIdx.x; i < (uint32_t)words; i += GATHER_T) out[o0 + i] = w[i];
+    __syncthreads();
   }
+}
+__global__ void __launch_bounds__(GATHER_T) k_gather(const unsigned long long *desc, unsigned long long n,
+                                                     const unsigned long long *goff, const uint32_t *arena,
+                                                     uint32_t ib, uint32_t ibm, uint32_t *out) {
+  gather_tiles(desc, n, [](unsigned long long v) { return v; }, goff, arena, ib, ibm, out);
 }
 
 // Per-game offsets relative to the game's first energy: game g owns entries
@@ -2406,19 +2431,37 @@ __global__ void k_sel_counts(const unsigned long long *desc, const uint32_t *sel
        i += (unsigned long long)gridDim.x * blockDim.x)
     cnt[i] = dcnt(desc[sel[i]]);
 }
-__global__ void k_sel_gather(const unsigned long long *desc, const uint32_t *sel, unsigned long long k,
-                             const unsigned long long *goff, const uint32_t *arena, uint32_t ib, uint32_t ibm,
-                             uint32_t *out) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const unsigned long long gw = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
-  const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-  for (unsigned long long i = gw; i < k; i += nw) {
-    const unsigned long long d = desc[sel[i]];
-    const uint32_t c = dcnt(d);
-    const unsigned long long go = goff[i];
-    for (uint32_t q = lane; q < c; q += 32u)
-      out[go + q] = dinl(d) ? ((uint32_t)(d >> (q * ib)) & ibm) : arena[doff(d) + q];
+__global__ void __launch_bounds__(GATHER_T) k_sel_gather(const unsigned long long *desc, const uint32_t *sel,
+                                                         unsigned long long k, const unsigned long long *goff,
+                                                         const uint32_t *arena, uint32_t ib, uint32_t ibm,
+                                                         uint32_t *out) {
+  gather_tiles(desc, k, [=](unsigned long long v) { return sel[v]; }, goff, arena, ib, ibm, out);
+}
+// A small selection in one launch of one block: offsets (k + 1) and, when they
+// fit in cap words, the energies, written to page-locked host memory.  cnt: k
+// words of scratch.
+constexpr uint32_t SEL_SMALL = 4096;
+__global__ void __launch_bounds__(SCAN_T) k_sel_small(const unsigned long long *desc, const uint32_t *sel, uint32_t k,
+                                                      const uint32_t *arena, uint32_t ib, uint32_t ibm,
+                                                      unsigned long long *h_off, uint32_t *h_data,
+                                                      unsigned long long cap) {
+  __shared__ unsigned long long ws[33];
+  unsigned long long carry = 0;
+  for (uint32_t t0 = 0; t0 < k; t0 += SCAN_T) {
+    const uint32_t i = t0 + threadIdx.x;
+    const unsigned long long d = i < k ? desc[sel[i]] : 0ull;
+    const uint32_t c = i < k ? dcnt(d) : 0u;
+    unsigned long long total;
+    const unsigned long long o = carry + block_excl_scan(c, ws, total);
+    if (i < k) {
+      h_off[i] = o;
+      if (o + c <= cap)
+        for (uint32_t q = 0; q < c; q++)
+          h_data[o + q] = dinl(d) ? ((uint32_t)(d >> (q * ib)) & ibm) : arena[doff(d) + q];
+    }
+    carry += total;
   }
+  if (threadIdx.x == 0) h_off[k] = carry;
 }
 
 __global__ void k_set_arena(Ctr *c, uint32_t *arena, unsigned long long cap, unsigned long long top) {
@@ -2574,6 +2617,39 @@ void HostBuf::reset() {
   pool.reset();
 }
 
+// The device half of a small upload in one launch (k_finish_cluster): what
+// finish_upload does in some 16 launches.
+struct FinishArgs {
+  uint32_t N, M, n_games, check_rows, any_init, std_reach;
+  unsigned long long n_reach;
+  uint32_t *row, *col;
+  const uint32_t *wt, *reach;
+  const uint8_t *flags;
+  const unsigned long long *node_base;  // n_games + 1 positions, edges, then sizes
+  uint32_t elements, ubits, umask;
+  unsigned long long *desc_init;
+  uint32_t *mark;
+  uint32_t mwords;  // both halves
+  uint32_t *abits, *rrow, *rcol, *cursor;
+  unsigned long long *cw;
+  uint32_t *h_err;  // page-locked
+  Ctr *ctr;         // its `pad` collects the error bits
+};
+// Uploads whose checks, reverse edges and restart are one launch each.  Median
+// of one comparison of two processes (12 in a row, 9.8 -> 8.6 ms) on one B200;
+// at 42,000 positions 16 blocks are slower than the whole chip's launches
+// (1.066 -> 1.09 ms a game), between the two sizes both measured alike.
+constexpr unsigned long long SMALL_UPLOAD_POSITIONS = 8192, SMALL_UPLOAD_EDGES = 65536;
+// The start of a solve in k_rounds_cluster's launch (desc == null: the launch
+// goes on from the control block): what solve_begin does in seven calls.
+struct BeginArgs {
+  const unsigned long long *desc_init;
+  const uint32_t *init_data, *reach;
+  unsigned long long init_total, n_reach, arena_cap;
+  uint32_t *arena;
+  uint32_t stamp, std_reach;
+};
+
 // Where rounds run inside one launch (k_rounds_cluster, k_solve_static), on one
 // B200, each figure the median of whole calls:
 // - uploads of up to CLUSTER_POSITIONS run all their rounds in cluster
@@ -2657,6 +2733,8 @@ struct DeviceGamesImpl {
     std::chrono::steady_clock::time_point t_start{};
   } prog;
   uint32_t frontier = ~0u;  // its size after the last step (unknown before the first)
+  uint32_t upload_launches = 0;  // counted with the first solve's (small uploads)
+  bool begin_pending = false;  // the next step's launch restarts the solve
   HostBuf hstep;            // page-locked: the control block and active flags read back by a step
   uint8_t *d_act = nullptr; // active flags on the device
   bool step_active = false;
@@ -2828,7 +2906,8 @@ void Engine::pool_put(void *p, size_t bytes) { st->pool.put(p, bytes); }
 static geq_status static_scratch(int device, unsigned char *&out);
 static geq_status cluster_setup(uint32_t &blocks);
 static geq_status launch_rounds_cluster(const Engine &E, const KParams &kp, bool generic, uint32_t max_rounds,
-                                        uint32_t limit);
+                                        uint32_t limit, const BeginArgs &begin);
+static geq_status launch_finish_cluster(const Engine &E, const FinishArgs &a, bool generic);
 
 geq_status Engine::create(int device, std::unique_ptr<Engine> &out) {
   int n = 0;
@@ -3246,6 +3325,42 @@ geq_status Engine::finish_upload(GamesPtr &dg, bool any_init, GamesPtr &out) {
   DeviceGamesImpl &D = *dg;
   const unsigned long long N = D.N, M = D.M, n_reach = D.n_reach;
   cudaStream_t S = s.stream;
+  const bool small = N && N <= SMALL_UPLOAD_POSITIONS && M <= SMALL_UPLOAD_EDGES && s.cluster > 1;
+  if (small) {
+    geq_status es = ensure_cnt(s, N + 1);
+    if (es) return es;
+    FinishArgs fa{};
+    fa.N = (uint32_t)N;
+    fa.M = (uint32_t)M;
+    fa.n_games = D.n_games;
+    fa.check_rows = D.rows_on_device ? 1u : 0u;
+    fa.any_init = any_init ? 1u : 0u;
+    fa.std_reach = D.std_reach ? 1u : 0u;
+    fa.n_reach = n_reach;
+    fa.row = D.row;
+    fa.col = D.col;
+    fa.wt = D.wt;
+    fa.flags = D.flags;
+    fa.reach = D.reach;
+    fa.node_base = D.d_node_base;
+    fa.elements = D.conf.elements;
+    fa.ubits = D.conf.update_bits();
+    fa.umask = D.conf.update_mask();
+    fa.desc_init = D.desc_init;
+    fa.mark = D.mark;
+    fa.mwords = (uint32_t)(2 * ((N + 31) / 32));
+    fa.abits = D.abits;
+    fa.rrow = D.rrow;
+    fa.rcol = D.rcol;
+    fa.cursor = s.cnt;
+    fa.cw = D.cw;
+    fa.h_err = &s.h_ctr->pad;
+    fa.ctr = D.ctr;
+    if ((es = launch_finish_cluster(*this, fa, D.generic))) return es;
+    D.upload_launches = 1;
+    CU(cudaStreamSynchronize(S));
+    return finish_params(dg, out);
+  }
   CU(cudaMemsetAsync(D.mark, 0, 2 * ((N + 31) / 32) * 4, S));
   CU(cudaMemsetAsync(s.d_err, 0, 4, S));
   const unsigned grid = (unsigned)std::max(1, n_sms * 8);
@@ -3295,6 +3410,14 @@ geq_status Engine::finish_upload(GamesPtr &dg, bool any_init, GamesPtr &out) {
 #endif
   s.pool.put(roff, (N + 1) * 8);
   CU(cudaGetLastError());
+  return finish_params(dg, out);
+}
+
+// The end of an upload: the checks' verdict, the kernels' parameters.
+geq_status Engine::finish_params(GamesPtr &dg, GamesPtr &out) {
+  State &s = *st;
+  DeviceGamesImpl &D = *dg;
+  const unsigned long long N = D.N, M = D.M;
   const uint32_t h_err = s.h_ctr->pad;
   if (h_err & 1u) return fail(GEQ_ERR_INVALID_INPUT, "Node index too high: a successor index is out of range");
   if (h_err & 2u) return fail(GEQ_ERR_INVALID_INPUT, "an edge update names no element or sets padding bits");
@@ -3469,14 +3592,26 @@ geq_status Engine::solve_begin(DeviceGamesImpl &dg) {
   pr = DeviceGamesImpl::Progress{};
   pr.t_start = std::chrono::steady_clock::now();
   dg.frontier = ~0u;
+  pr.launches = dg.upload_launches;
+  dg.upload_launches = 0;
+  CU(cudaEventRecord(s.ev0, S));
+  if (dg.next_stamp > 0xF0000000u) dg.next_stamp = 1;
+  dg.kp.cw = (tuning.flags & GEQ_TUNE_NO_EDGE_PAIRS) ? nullptr : dg.cw;
+  dg.kp.missing = nullptr;
+  // an upload whose rounds run in cluster launches is restarted by the first
+  dg.begin_pending = dg.N && dg.N <= SMALL_UPLOAD_POSITIONS && dg.off_ranges.empty() &&
+                     !(tuning.flags & (GEQ_TUNE_NO_GRAPH | GEQ_TUNE_PROFILE | GEQ_TUNE_READY));
+  return dg.begin_pending ? GEQ_OK : begin_launches(dg);
+}
+geq_status Engine::begin_launches(DeviceGamesImpl &dg) {
+  State &s = *st;
+  cudaStream_t S = s.stream;
+  DeviceGamesImpl::Progress &pr = dg.prog;
   // restart from the uploaded initial state
   const int a0 = dg.arena_cur;
-  CU(cudaEventRecord(s.ev0, S));
   if (dg.N) CU(cudaMemcpyAsync(dg.desc, dg.desc_init, dg.N * 8, cudaMemcpyDeviceToDevice, S));
   CU(cudaMemcpyAsync(dg.arena[a0], dg.init_data, dg.init_total * 4, cudaMemcpyDeviceToDevice, S));
-  if (dg.next_stamp > 0xF0000000u) dg.next_stamp = 1;
   CU(cudaMemsetAsync(dg.mark, 0, 2ull * dg.kp.mwords * 4, S));
-  dg.kp.cw = (tuning.flags & GEQ_TUNE_NO_EDGE_PAIRS) ? nullptr : dg.cw;
   // GEQ_TUNE_READY: defenders wait for their successors' lists (counted per
   // defender, set up at the first such solve); else every predecessor of a
   // changed position is pushed, as the reference's visit lists do
@@ -3646,10 +3781,21 @@ geq_status Engine::step_enqueue(DeviceGamesImpl &dg, bool active) {
   // small uploads, and the rounds of medium ones whose frontier has become
   // small, run inside one launch of a cluster of blocks
   const bool whole = dg.N <= CLUSTER_POSITIONS;
+  if (dg.begin_pending && !(use_graph && whole)) {  // the tuning changed since solve_begin
+    dg.begin_pending = false;
+    geq_status g = begin_launches(dg);
+    if (g) return g;
+  }
   const bool cluster = use_graph && (whole || (dg.N <= CLUSTER_POSITIONS_TAIL && dg.frontier <= CLUSTER_FRONTIER));
   if (cluster) {
+    BeginArgs begin{};
+    if (dg.begin_pending) {
+      begin = BeginArgs{dg.desc_init, dg.init_data, dg.reach, dg.init_total, dg.n_reach, dg.arena_cap[dg.arena_cur],
+                        dg.arena[dg.arena_cur], dg.next_stamp, dg.std_reach ? 1u : 0u};
+      dg.begin_pending = false;
+    }
     geq_status g = launch_rounds_cluster(*this, dg.kp, dg.generic, active ? CLUSTER_ROUNDS_SERVING : CLUSTER_ROUNDS,
-                                         whole ? ~0u : 2 * CLUSTER_FRONTIER);
+                                         whole ? ~0u : 2 * CLUSTER_FRONTIER, begin);
     if (g) return g;
     pr.launches++;
   } else if (use_graph) {
@@ -3730,11 +3876,8 @@ geq_status Engine::solve_step(DeviceGamesImpl &dg, bool &done) {
 }
 
 geq_status Engine::solve_stats(DeviceGamesImpl &dg, geq_solve_stats *stats) {
-  State &s = *st;
-  cudaStream_t S = s.stream;
-  CU(cudaMemcpyAsync(s.h_ctr, dg.ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, S));
-  CU(cudaStreamSynchronize(S));
-  const Ctr c = *s.h_ctr;
+  // the counters as the last finished step read them back
+  const Ctr c = dg.hstep.p ? *(const Ctr *)dg.hstep.p : Ctr{};
   if (stats) {
     *stats = geq_solve_stats{};
     stats->rounds = c.rounds;
@@ -3754,13 +3897,16 @@ geq_status Engine::solve(DeviceGamesImpl &dg, geq_solve_stats *stats) {
   cudaStream_t S = s.stream;
   geq_status st_ = solve_begin(dg);
   if (st_) return st_;
-  for (bool done = false; !done;)
-    if ((st_ = solve_step(dg, done))) return st_;
-  CU(cudaEventRecord(s.ev1, S));
+  for (bool done = false; !done;) {
+    if ((st_ = step_enqueue(dg, false))) return st_;
+    CU(cudaEventRecord(s.ev1, S));
+    const uint8_t *active = nullptr;
+    if ((st_ = sync()) || (st_ = step_finish(dg, done, active))) return st_;
+  }
   if ((st_ = solve_stats(dg, stats))) return st_;
 #if GEQ_PATH_PROFILE
   {
-    const Ctr c = *s.h_ctr;
+    const Ctr c = *(const Ctr *)dg.hstep.p;
     std::fprintf(stderr, "GEQ_PROF");
     for (int i = 0; i < 32; i++) std::fprintf(stderr, " %llu", c.prof[i]);
     std::fprintf(stderr, "\n");
@@ -4019,6 +4165,22 @@ geq_status run_batch_pipelined(int device, Engine &ea, Engine &eb, std::vector<G
   return GEQ_OK;
 }
 
+// A solution's per-game bases and offsets from the selection's offsets.
+static void selected_layout(const unsigned long long *off, const std::vector<uint32_t> &count, geq_solution &sol) {
+  const uint32_t G = (uint32_t)count.size();
+  sol.n_vertices.assign(count.begin(), count.end());
+  sol.offsets_base.resize(G);
+  sol.data_base.resize(G);
+  sol.offsets.clear();
+  unsigned long long k = 0;
+  for (uint32_t g = 0; g < G; g++) {
+    sol.offsets_base[g] = sol.offsets.size();
+    sol.data_base[g] = off[k];
+    for (uint32_t i = 0; i <= count[g]; i++) sol.offsets.push_back(off[k + i] - off[k]);
+    k += count[g];
+  }
+}
+
 geq_status Engine::download_selected(DeviceGamesImpl &dg, const std::vector<uint32_t> &first,
                                      const std::vector<uint32_t> &count, geq_solution &sol) {
   State &s = *st;
@@ -4029,6 +4191,27 @@ geq_status Engine::download_selected(DeviceGamesImpl &dg, const std::vector<uint
     for (uint32_t i = 0; i < count[g]; i++) sel.push_back((uint32_t)(dg.node_base[g] + first[g] + i));
   const unsigned long long K = sel.size();
   unsigned long long launches = 0;
+  if (K && K <= SEL_SMALL) {
+    // one launch and one wait: offsets, energies and the selection itself are
+    // page-locked memory the kernel reads and writes
+    HostBuf off_b, data_b, sel_b;
+    const unsigned long long cap = 8 * K + 1024;
+    if (off_b.alloc(s.hpool, (K + 1) * 8) && data_b.alloc(s.hpool, cap * 4) && sel_b.alloc(s.hpool, K * 4) &&
+        off_b.pool && data_b.pool && sel_b.pool) {
+      std::memcpy(sel_b.p, sel.data(), K * 4);
+      const unsigned long long *off = (const unsigned long long *)off_b.p;
+      k_sel_small<<<1, SCAN_T, 0, S>>>(dg.desc, (const uint32_t *)sel_b.p, (uint32_t)K, dg.arena[dg.arena_cur],
+                                       dg.kp.ib, dg.kp.ibm, (unsigned long long *)off_b.p, (uint32_t *)data_b.p, cap);
+      CU(cudaGetLastError());
+      CU(cudaStreamSynchronize(S));
+      if (off[K] <= cap) {
+        sol.energy_size = 1;
+        sol.data.assign((const uint32_t *)data_b.p, (const uint32_t *)data_b.p + off[K]);
+        selected_layout(off, count, sol);
+        return GEQ_OK;
+      }
+    }
+  }
   geq_status a = ensure_cnt(s, K + 1);
   if (a) return a;
   uint32_t *d_sel = (uint32_t *)s.pool.get(std::max<unsigned long long>(K, 1) * 4);
@@ -4053,18 +4236,7 @@ geq_status Engine::download_selected(DeviceGamesImpl &dg, const std::vector<uint
   s.pool.put(d_sel, std::max<unsigned long long>(K, 1) * 4);
   s.pool.put(goff, (K + 1) * 8);
   s.pool.put(out, std::max<unsigned long long>(total, 1) * 4);
-  sol.n_vertices.assign(count.begin(), count.end());
-  sol.offsets_base.resize(G);
-  sol.data_base.resize(G);
-  sol.offsets.clear();
-  sol.offsets.reserve(K + G);
-  unsigned long long k = 0;
-  for (uint32_t g = 0; g < G; g++) {
-    sol.offsets_base[g] = sol.offsets.size();
-    sol.data_base[g] = off[k];
-    for (uint32_t i = 0; i <= count[g]; i++) sol.offsets.push_back(off[k + i] - off[k]);
-    k += count[g];
-  }
+  selected_layout(off.data(), count, sol);
   return GEQ_OK;
 }
 
@@ -4291,16 +4463,51 @@ __device__ void group_rounds(const KParams &p, Ctr *c, const Group &g, RoundStat
 // Rounds of an upload by one cluster: the state is taken from the control
 // block and left there as k_commit / k_ffill leave it.
 template <class Cd>
-__global__ void __launch_bounds__(CT, 1) k_rounds_cluster(const KParams p, uint32_t max_rounds, uint32_t limit) {
+__global__ void __launch_bounds__(CT, 1) k_rounds_cluster(const KParams p, uint32_t max_rounds, uint32_t limit,
+                                                          const BeginArgs a) {
   extern __shared__ uint32_t dsm[];
   __shared__ uint32_t wsum[2 * CW + 2], s_flags;
   Ctr *c = p.ctr;
   const Group g = this_group();
-  RoundState st{c->cur, c->fsize[c->cur], c->stamp, 0u};
-  if (c->halt) st.fs = 0u;
-  const bool idle = st.fs == 0u || st.fs > limit;
-  g.sync();  // every block has read the state
-  if (idle) return;
+  RoundState st{0u, 0u, a.stamp, 0u};
+  if (a.desc_init) {
+    // restart from the uploaded initial state; the initial visit lists are the
+    // predecessors of the positions to reach (energygame.rs:1461-1465)
+    const uint32_t lane = threadIdx.x & 31u;
+    if (g.tid == 0) {
+      Ctr h{};
+      h.arena = a.arena;
+      h.arena_cap = a.arena_cap;
+      h.arena_top = a.init_total;
+      h.stamp = a.stamp;
+      *c = h;
+    }
+    for (unsigned long long v = g.tid; v < p.n_nodes; v += g.threads) p.desc[v] = a.desc_init[v];
+    for (unsigned long long i = g.tid; i < a.init_total; i += g.threads) a.arena[i] = a.init_data[i];
+    for (uint32_t i = g.tid; i < 2u * p.mwords; i += g.threads) p.mark[i] = 0u;
+    g.sync();
+    const unsigned long long n_src = a.std_reach ? p.n_nodes : a.n_reach;
+    uint32_t *sm = dsm + (threadIdx.x >> 5) * CWARP_WORDS;
+    for (unsigned long long b0 = (unsigned long long)(g.tid >> 5) * 32u; b0 < n_src; b0 += g.threads) {
+      const unsigned long long i = b0 + lane;
+      bool f = false;
+      uint32_t v = 0;
+      if (i < n_src) {
+        v = a.std_reach ? (uint32_t)i : a.reach[i];
+        f = a.std_reach ? !(p.flags[v] & 1u) && p.row[v] == p.row[v + 1ull] : true;
+      }
+      push_preds_warp(p, c, sm, v, f, a.stamp, lane);
+    }
+    g.sync();
+    st.fs = group_fill(p, c, g, a.stamp, p.front0, wsum);
+    g.sync();
+  } else {
+    st = RoundState{c->cur, c->fsize[c->cur], c->stamp, 0u};
+    if (c->halt) st.fs = 0u;
+    const bool idle = st.fs == 0u || st.fs > limit;
+    g.sync();  // every block has read the state
+    if (idle) return;
+  }
   group_rounds<Cd>(p, c, g, st, max_rounds, limit, dsm, wsum, &s_flags);
   if (g.tid == 0) {
     c->fsize[0] = st.cur ? 0u : st.fs;
@@ -4315,6 +4522,87 @@ __global__ void __launch_bounds__(CT, 1) k_rounds_cluster(const KParams p, uint3
     c->next_push = 0u;
     if (c->overflow) c->halt = 1u;
   }
+}
+
+// finish_upload for a small upload: row checks, rows and columns into the
+// global id space, weight checks, edge pairs, initial lists, reverse CSR and
+// the attacker bitmap.  Launches of their own cost each of those passes more
+// than its work.
+template <class T, class F>
+__device__ void block_excl_scan_n(unsigned long long n, F cnt, T *out, unsigned long long *ws);
+template <class Cd>
+__global__ void __launch_bounds__(CT, 1) k_finish_cluster(const FinishArgs a) {
+  __shared__ unsigned long long ws[34];
+  const Group g = this_group();
+  const unsigned long long *nb = a.node_base, *eb = nb + (a.n_games + 1), *gn = eb + (a.n_games + 1);
+  uint32_t *err = &a.ctr->pad;
+  if (g.tid == 0) *err = 0u;
+  for (uint32_t v = g.tid; v < a.N; v += g.threads) {
+    a.cursor[v] = 0u;
+    if (!a.any_init) a.desc_init[v] = 0ull;
+  }
+  for (uint32_t i = g.tid; i < a.mwords; i += g.threads) a.mark[i] = 0u;
+  g.sync();
+  uint32_t bad = 0;
+  if (a.check_rows)
+    for (uint32_t v = g.tid; v < a.N; v += g.threads) {
+      const uint32_t k = game_of(nb, a.n_games, v);
+      const uint32_t r = a.row[v];
+      const unsigned long long next = (v + 1ull < nb[k + 1]) ? a.row[v + 1] : (eb[k + 1] - eb[k]);
+      if ((v == nb[k] && r != 0u) || r > next) bad |= 4u;
+    }
+  g.sync();
+  if (a.n_games > 1)
+    for (uint32_t v = g.tid; v < a.N; v += g.threads) a.row[v] += (uint32_t)eb[game_of(nb, a.n_games, v)];
+  for (uint32_t k = g.tid; k < a.M; k += g.threads) {
+    const uint32_t q = a.n_games > 1 ? game_of(eb, a.n_games, k) : 0u;
+    uint32_t w = a.col[k];
+    if (w >= gn[q]) bad |= 1u;
+    w += (uint32_t)nb[q];
+    a.col[k] = w;
+    if (w < a.N) atomicAdd(&a.cursor[w], 1u);
+    else bad |= 1u;
+    const uint32_t u = a.wt[k];
+    if (a.elements * a.ubits < 32u && (u >> (a.elements * a.ubits)) != 0u) bad |= 2u;
+    for (uint32_t i = 0; i < a.elements; i++)
+      if (((u >> (i * a.ubits)) & a.umask) > a.elements + 1u) bad |= 2u;
+    a.cw[k] = (unsigned long long)w | ((unsigned long long)Cd::pack_edge(u) << 32);
+  }
+  if (bad) atomicOr(err, bad);
+  for (uint32_t i = g.tid; i < (a.N + 31u) / 32u; i += g.threads) {
+    uint32_t w = 0;
+    for (uint32_t k = 0; k < 32u; k++) {
+      const uint32_t v = i * 32u + k;
+      if (v < a.N && (a.flags[v] & 1u)) w |= 1u << k;
+    }
+    a.abits[i] = w;
+  }
+  g.sync();
+  if (g.rank == 0)
+    block_excl_scan_n<uint32_t>(a.N, [&](unsigned long long v) { return a.cursor[v]; }, a.rrow, ws);
+  if (!a.any_init) {
+    if (a.std_reach) {
+      for (uint32_t v = g.tid; v < a.N; v += g.threads)
+        if (!(a.flags[v] & 1u) && a.row[v] == a.row[v + 1]) a.desc_init[v] = inl_hdr(1u);
+    } else {
+      for (unsigned long long i = g.tid; i < a.n_reach; i += g.threads) a.desc_init[a.reach[i]] = inl_hdr(1u);
+    }
+  }
+  g.sync();
+  for (uint32_t v = g.tid; v < a.N; v += g.threads) a.cursor[v] = a.rrow[v];
+  g.sync();
+  // (an upload that failed a check is refused: its rows may name any range)
+  const uint32_t n_fill = *(volatile uint32_t *)err ? 0u : a.N;
+  for (uint32_t v = g.tid; v < n_fill; v += g.threads) {
+    const uint32_t e = min(a.row[v + 1], a.M);
+    for (uint32_t k = a.row[v]; k < e; k++) {
+      const uint32_t w = a.col[k];
+      if (w >= a.N) continue;
+      const uint32_t pos = atomicAdd(&a.cursor[w], 1u);
+      if (pos < a.M) a.rcol[pos] = v;
+    }
+  }
+  if (g.tid == 0) *a.h_err = *(volatile uint32_t *)err;
 }
 
 // out[v] = sum of cnt(u) for u < v, out[n] = the total; one block.  ws: 34
@@ -4484,6 +4772,8 @@ static cudaError_t cluster_attrs(F *f) {
 static geq_status cluster_setup(uint32_t &blocks) {
   CU(cluster_attrs(k_rounds_cluster<CodecStd>));
   CU(cluster_attrs(k_rounds_cluster<CodecGen>));
+  CU(cluster_attrs(k_finish_cluster<CodecStd>));
+  CU(cluster_attrs(k_finish_cluster<CodecGen>));
   CU(cluster_attrs(k_solve_static<CodecStd>));
   CU(cluster_attrs(k_solve_static<CodecGen>));
   for (blocks = 16; blocks > 1; blocks /= 2) {
@@ -4506,10 +4796,16 @@ static geq_status cluster_setup(uint32_t &blocks) {
   return GEQ_OK;
 }
 static geq_status launch_rounds_cluster(const Engine &E, const KParams &kp, bool generic, uint32_t max_rounds,
-                                        uint32_t limit) {
+                                        uint32_t limit, const BeginArgs &begin) {
   const Engine::State &s = *E.st;
-  CU(generic ? launch_cluster(k_rounds_cluster<CodecGen>, s.cluster, CW, s.stream, kp, max_rounds, limit)
-             : launch_cluster(k_rounds_cluster<CodecStd>, s.cluster, CW, s.stream, kp, max_rounds, limit));
+  CU(generic ? launch_cluster(k_rounds_cluster<CodecGen>, s.cluster, CW, s.stream, kp, max_rounds, limit, begin)
+             : launch_cluster(k_rounds_cluster<CodecStd>, s.cluster, CW, s.stream, kp, max_rounds, limit, begin));
+  return GEQ_OK;
+}
+static geq_status launch_finish_cluster(const Engine &E, const FinishArgs &a, bool generic) {
+  const Engine::State &s = *E.st;
+  CU(generic ? launch_cluster(k_finish_cluster<CodecGen>, s.cluster, CW, s.stream, a)
+             : launch_cluster(k_finish_cluster<CodecStd>, s.cluster, CW, s.stream, a));
   return GEQ_OK;
 }
 static geq_status launch_solve_static(const KParams &kp, const StaticArgs &sa, bool generic, uint32_t blocks,

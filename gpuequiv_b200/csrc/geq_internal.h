@@ -275,6 +275,8 @@ class Engine {
   geq_status clear_off_ranges(DeviceGamesImpl &dg, uint32_t stamp);
   geq_status alloc_work(DeviceGamesImpl &D, bool any_init);
   geq_status finish_upload(GamesPtr &dg, bool any_init, GamesPtr &out);
+  geq_status finish_params(GamesPtr &dg, GamesPtr &out);
+  geq_status begin_launches(DeviceGamesImpl &dg);
 };
 
 // The games of jobs L[j] with start positions Attack(p[t], {q[t]}) for t in
