@@ -376,6 +376,7 @@ template <int ES>
 struct SWarp {
   uint32_t A[SCAP * ES], B[SCAP * ES];  // members
   uint32_t Y[32 * ES];                  // a chunk of updated energies
+  uint32_t Q[64 * ES];                  // suprema that wait to be inserted
   uint32_t inc[32];
   uint8_t fl[SCAP];                     // own energy (attacker tie rule)
 };
@@ -566,7 +567,23 @@ __device__ bool solve_es(const P &p, uint32_t slot, SWarp<ES> &s, uint32_t lane,
       const unsigned long long d = p.desc[p.col[k]];
       const uint32_t *u = p.wt + (unsigned long long)k * p.us;
       by += esb * dcnt(d);
-      uint32_t nb = 0;
+      uint32_t nb = 0, nq = 0;
+      auto drain = [&](uint32_t c) {  // the first c waiting suprema go in
+        __syncwarp();
+        uint32_t z[ES] = {}, r[ES] = {};
+#pragma unroll
+        for (int w = 0; w < ES; w++) {
+          if (lane < c) z[w] = s.Q[lane * ES + w];
+          if (lane + c < nq) r[w] = s.Q[(lane + c) * ES + w];
+        }
+        __syncwarp();
+        if (lane + c < nq) {
+#pragma unroll
+          for (int w = 0; w < ES; w++) s.Q[lane * ES + w] = r[w];
+        }
+        nq -= c;
+        return insert32<ES>(p, B, s.fl, nb, z, lane < c, false, lane);
+      };
       for (uint32_t q0 = 0; q0 < dcnt(d); q0 += 32u) {
         const uint32_t ny = min(32u, dcnt(d) - q0);
         uint32_t x[ES] = {};
@@ -592,20 +609,72 @@ __device__ bool solve_es(const P &p, uint32_t slot, SWarp<ES> &s, uint32_t lane,
           for (int w = 0; w < ES; w++) s.Y[lane * ES + w] = x[w];
         }
         __syncwarp();
+        if (ny * n == 1u) {  // nothing to leave out
+          if (nq && !drain(nq)) return false;
+          uint32_t z[ES];
+#pragma unroll
+          for (int w = 0; w < ES; w++) z[w] = max_w(A[w], s.Y[w], p.sw);
+          if (!insert32<ES>(p, B, s.fl, nb, z, lane == 0, false, lane)) return false;
+          continue;
+        }
+        // Where a member lies at or below y, y itself is a supremum and every
+        // other one with y lies above it; likewise where an energy of this
+        // chunk lies at or below a member.  Only what is left is inserted:
+        // conf {30, 3}, 12,000 positions 8.1 -> 6.3 ms, {16, 7}, 20,000 positions
+        // 4.2 -> 3.5 ms on one B200.
+        bool hy = lane >= ny;
+        uint32_t ha = 0;  // bit j: member 32j + lane
+        for (uint32_t m = 0; m < n && !__all_sync(FULL, hy); m++) {
+          uint32_t mv[ES];
+#pragma unroll
+          for (int w = 0; w < ES; w++) mv[w] = A[m * ES + w];
+          hy = hy || leq_es<ES>(mv, x, p.sw);
+        }
+        const uint32_t hits = __ballot_sync(FULL, hy);
+        for (uint32_t m = lane; m < n; m += 32u) {
+          uint32_t mv[ES], yv[ES];
+#pragma unroll
+          for (int w = 0; w < ES; w++) mv[w] = A[m * ES + w];
+          bool h = false;
+          for (uint32_t q = 0; q < ny && !h; q++) {
+#pragma unroll
+            for (int w = 0; w < ES; w++) yv[w] = s.Y[q * ES + w];
+            h = leq_es<ES>(yv, mv, p.sw);
+          }
+          if (h) ha |= 1u << (m >> 5);
+        }
+        __syncwarp();
+        uint32_t yq = lane / n, am = lane - yq * n;
         for (uint32_t i0 = 0; i0 < ny * n; i0 += 32u) {
-          const uint32_t i = i0 + lane;
-          const bool valid = i < ny * n;
+          const bool valid = i0 + lane < ny * n;
+          const uint32_t hm = __shfl_sync(FULL, ha, am & 31u);
+          bool keep = valid;
           uint32_t z[ES] = {};
           if (valid) {
-            const uint32_t yq = i / n, am = i - yq * n;
+            bool ey = true, ea = true;  // the supremum is y, is the member
 #pragma unroll
-            for (int w = 0; w < ES; w++) z[w] = max_w(A[am * ES + w], s.Y[yq * ES + w], p.sw);
+            for (int w = 0; w < ES; w++) {
+              const uint32_t av = A[am * ES + w], yv = s.Y[yq * ES + w];
+              z[w] = max_w(av, yv, p.sw);
+              ey = ey && z[w] == yv;
+              ea = ea && z[w] == av;
+            }
+            keep = (ey || !((hits >> yq) & 1u)) && (ea || !((hm >> (am >> 5)) & 1u));
           }
-          if (!insert32<ES>(p, B, s.fl, nb, z, valid, false, lane)) return false;
+          const uint32_t bal = __ballot_sync(FULL, keep);
+          if (keep) {
+            const uint32_t d = nq + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+            for (int w = 0; w < ES; w++) s.Q[d * ES + w] = z[w];
+          }
+          nq += (uint32_t)__popc(bal);
+          if (nq >= 32u && !drain(32u)) return false;
+          for (am += 32u; am >= n; am -= n) yq++;
         }
         __syncwarp();
       }
       if (k != e0) {
+        if (nq && !drain(nq)) return false;
         uint32_t *t = A;
         A = B;
         B = t;

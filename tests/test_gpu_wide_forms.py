@@ -119,3 +119,29 @@ def test_game_sizes(geq, ctx, conf, n):
     es = geq.EnergyConf(*conf).energy_size()
     run_both(geq, ctx, conf, row, col, update_words(geq, conf, codes), att, reach, offs,
              np.zeros((int(offs[-1]), es), np.uint32))
+
+
+@pytest.mark.parametrize("conf", [(2, 65535), (30, 3), (50, 3), (1, 0xFFFFFFFF)])
+@pytest.mark.parametrize("na,nb", [(1, 1), (1, 40), (40, 1), (5, 7), (31, 33), (33, 32), (2, 128)])
+def test_suprema_left_out(geq, ctx, conf, na, nb):
+    """A defender over lists that share members, hold energies above and below
+    the other's, and none comparable: products of which most, some or no
+    suprema are left out before they are inserted."""
+    rng = np.random.default_rng(1000 * na + nb)
+    el, mx = conf
+    top = min(mx, 3)
+    for kind in ("shared", "above", "apart"):
+        a = rng.integers(0, top + 1, (na, el)).astype(np.uint64)
+        b = rng.integers(0, top + 1, (nb, el)).astype(np.uint64)
+        k = min(na, nb)
+        if kind == "shared":
+            b[:k:2] = a[:k:2]
+        elif kind == "above":  # every second energy above or below one of the other list
+            b[:k:4] = np.minimum(a[:k:4] + rng.integers(0, 2, a[:k:4].shape).astype(np.uint64), top)
+            a[2:k:4] = np.minimum(b[2:k:4] + rng.integers(0, 2, b[2:k:4].shape).astype(np.uint64), top)
+        lists = [pack(geq, conf, a), pack(geq, conf, b)]
+        row = np.array([0, 1, 3, 3, 3], np.uint32)
+        col = np.array([1, 2, 3], np.uint32)
+        offs = np.array([0, 0, 0, na, na + nb], np.uint64)
+        run_both(geq, ctx, conf, row, col, update_words(geq, conf, np.zeros((3, el), np.uint32)),
+                 np.array([1, 0, 1, 1], np.uint8), np.array([2, 3], np.uint32), offs, np.concatenate(lists))
