@@ -26,6 +26,14 @@
 //     (attackers first, each kind in position order).
 //   * Rounds are launched as CUDA graphs of several rounds each; the host
 //     reads one small counter block per graph launch to detect termination.
+//   * Uploads of up to 32,768 positions, and the rounds of uploads of up to a
+//     million whose frontier has become small, run inside one launch of a
+//     cluster of 16 blocks (k_rounds_cluster), a lone small game from upload
+//     to result (k_solve_static): their rounds are shorter than the launches
+//     of four kernels.
+//   * k_round spreads a small frontier over all its warps (lanes_solve: the
+//     positions of a warp worked on together), and long predecessor lists are
+//     cut into parts for k_round_big's warps (pushq).
 //
 // Results are identical to the reference's: the same positions are recomputed
 // in the same rounds from the same inputs.  The one scheduling difference is
@@ -4243,10 +4251,11 @@ geq_status Engine::download_selected(DeviceGamesImpl &dg, const std::vector<uint
 // ---- allocation-free solve of one game (geq_energy_game_run_static) -------
 // All device memory of this solve is one file-scope array: the game, its
 // reverse CSR, descriptors, frontiers, control block and energy arena.  One
-// block of BLOCK threads runs the whole solve in one launch -- validation,
-// reverse CSR, initialisation, the rounds (the position routines of k_round,
-// with block barriers between a round and its commit) and the gather of the
-// result lists -- so the call allocates nothing and launches one kernel.
+// block runs the whole solve in one launch -- validation, reverse CSR,
+// initialisation, the rounds (the position routines of k_round, with barriers
+// between a round and its commit) and the gather of the result lists -- so the
+// call allocates nothing and launches one kernel.  solve_small runs the same
+// kernel over a cluster of blocks, in a pooled block of memory.
 static __device__ __align__(256) unsigned char g_static_scratch[GEQ_STATIC_SCRATCH_BYTES];
 
 struct StaticArgs {

@@ -2,7 +2,9 @@
 // minimisation (refine.cuh) on the CUDA stream of a context:
 // GameBuild::compare (src/gamebuild.rs:165-170) for a batch of (LTS, p, q)
 // jobs, one breadth-first level per pass over the level kernels (all levels
-// inside one CUDA graph WHILE node), results either copied back as one CSR
+// inside one CUDA graph WHILE node; levels of up to 4,096 positions, and the
+// minimisation of small batches, inside one launch of a cluster of blocks),
+// results either copied back as one CSR
 // game graph per job (geq_game_build_compare_batch) or handed to the solver
 // on the device (build_and_upload, used by geq_compare_batch, the serving
 // loop's queries and geq_equivalences); and

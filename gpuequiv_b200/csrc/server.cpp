@@ -223,7 +223,7 @@ geq_status retire(Engine &e, Session &ss, const std::vector<uint32_t> &games, st
 }
 
 // Games of one conf with a thermometer codec: a lone small game in one
-// launch of the one-block solver, else an upload that becomes a session.  An
+// launch (Engine::solve_small), else an upload that becomes a session.  An
 // upload of several games that fails is retried game by game, so that a
 // malformed game fails alone.
 void start_games(Engine &e, std::vector<Request *> &batch, uint64_t footprint,
