@@ -53,13 +53,13 @@ constexpr unsigned long long CNT_MASK = (1ull << CNT_BITS) - 1ull;
 
 struct Ctr {
   unsigned long long arena_top;  // energies in use
-  unsigned long long rounds;     // completed by k_wide_cluster
+  unsigned long long rounds;     // completed by k_wide_rounds
   unsigned long long positions, edges, bytes;
   uint32_t next_slot;   // slots handed out to warps
   uint32_t n_ovf;       // slots whose antichain outgrew the warp scratch
   uint32_t arena_full;  // a new list found no arena space
   uint32_t next_size;   // size of the next frontier
-  uint32_t flip;        // k_wide_cluster: 1 when `next` holds the frontier
+  uint32_t flip;        // k_wide_rounds: 1 when `next` holds the frontier
   uint32_t pad;
 };
 
@@ -749,17 +749,21 @@ __global__ void __launch_bounds__(BLOCK_T) k_wide_round_es(const P p) {
   }
 }
 
-// Rounds inside one launch of a cluster of blocks, for games of some ten
-// thousand positions: three barriers a round in place of three launches, four
-// fills, two read-backs and the waits for them.  Leaves before the commit of a
-// round that met a full arena or antichains beyond SCAP members, for the host
-// to finish that round.
+// Rounds inside one launch, four barriers a round in place of three launches,
+// four fills, two read-backs and the waits for them: of a cluster of blocks
+// (GRID = false) for small games, whose rounds are shorter than a barrier of
+// the whole device, else of a block per SM (a cooperative launch).  Leaves
+// before the commit of a round that met a full arena or antichains beyond SCAP
+// members, for the host to finish that round.
 constexpr uint32_t CWARPS = 16, CTHREADS = 32 * CWARPS;
-template <int ES>
-__global__ void __launch_bounds__(CTHREADS, 1) k_wide_cluster(P p, uint32_t fs, uint32_t max_rounds) {
+template <int ES, bool GRID>
+__global__ void __launch_bounds__(CTHREADS, 1) k_wide_rounds(P p, uint32_t fs, uint32_t max_rounds) {
   extern __shared__ __align__(16) unsigned char dsm[];
-  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-  const uint32_t rank = cl.block_rank(), blocks = cl.num_blocks();
+  const uint32_t rank = blockIdx.x, blocks = gridDim.x;  // one cluster, or the grid
+  auto sync = [] {
+    if constexpr (GRID) cooperative_groups::this_grid().sync();
+    else cooperative_groups::this_cluster().sync();
+  };
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   SWarp<ES> &s = ((SWarp<ES> *)dsm)[warp];
   const uint32_t gw = warp * blocks + rank, warps = blocks * CWARPS;
@@ -784,7 +788,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wide_cluster(P p, uint32_t fs, 
       }
       __syncwarp();
     }
-    cl.sync();
+    sync();
     stop = *(volatile uint32_t *)&c->n_ovf != 0u || *(volatile uint32_t *)&c->arena_full != 0u;
     if (stop) break;
     for (uint32_t k = tid; k < fs; k += threads) {
@@ -801,7 +805,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wide_cluster(P p, uint32_t fs, 
       c->next_slot = 0u;
       c->next_size = 0u;
     }
-    cl.sync();
+    sync();
     for (uint32_t w = tid; w < p.mwords; w += threads) {
       uint32_t b = p.mark[w];
       if (!b) continue;
@@ -809,14 +813,14 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wide_cluster(P p, uint32_t fs, 
       uint32_t at = atomicAdd(&c->next_size, (uint32_t)__popc(b));
       for (; b; b &= b - 1u) next[at++] = w * 32u + (uint32_t)__ffs((int)b) - 1u;
     }
-    cl.sync();
+    sync();
     fs = *(volatile uint32_t *)&c->next_size;
     uint32_t *t = front;
     front = next;
     next = t;
     flip ^= 1u;
     rounds++;
-    cl.sync();  // everyone has read the size
+    sync();  // everyone has read the size
   }
   if (lane == 0 && pos) {
     atomicAdd(&c->positions, pos);
@@ -828,7 +832,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wide_cluster(P p, uint32_t fs, 
     c->next_size = fs;
     c->flip = flip;
   }
-  cl.sync();
+  sync();
 }
 
 // publish the round's lists and mark the predecessors of changed positions
@@ -927,8 +931,8 @@ struct Bufs {
 template <int ES>
 static uint32_t cluster_setup_es() {
   const size_t smem = sizeof(SWarp<ES>) * CWARPS;
-  if (cudaFuncSetAttribute(k_wide_cluster<ES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_wide_cluster<ES>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+  if (cudaFuncSetAttribute(k_wide_rounds<ES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_wide_rounds<ES, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -944,7 +948,7 @@ static uint32_t cluster_setup_es() {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_wide_cluster<ES>, &cfg) == cudaSuccess && n > 0) return b;
+    if (cudaOccupancyMaxActiveClusters(&n, k_wide_rounds<ES, false>, &cfg) == cudaSuccess && n > 0) return b;
     cudaGetLastError();
   }
   return 0;
@@ -971,15 +975,54 @@ static cudaError_t launch_cluster_es(const P &p, uint32_t blocks, uint32_t fs, u
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_wide_cluster<ES>, p, fs, max_rounds);
+  return cudaLaunchKernelEx(&cfg, k_wide_rounds<ES, false>, p, fs, max_rounds);
 }
-// Games of up to so many positions run their rounds inside cluster launches.
-// Median per call on one B200, one warp per position in global scratch / these kernels without and
-// with the cluster, 8, 16 and 24 warps a block: conf {30, 3}, 12,000 positions
-// 21.2 / 10.0 / 8.6, 8.1, 8.6 ms; 300 positions 1.42 / 1.11 / 0.49, 0.50, 0.51
-// ms; {16, 7}, 20,000 positions 6.1 / 5.2 / 5.0, 4.2, 4.2 ms.
-constexpr uint32_t WIDE_CLUSTER_POSITIONS = 65536;
-constexpr uint32_t WIDE_CLUSTER_ROUNDS = 256;       // per launch
+// The same over the whole device: blocks of a cooperative launch, 0: none.
+template <int ES>
+static uint32_t grid_setup_es(int device) {
+  const size_t smem = sizeof(SWarp<ES>) * CWARPS;
+  int sms = 0, coop = 0, per = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop ||
+      cudaFuncSetAttribute(k_wide_rounds<ES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_wide_rounds<ES, true>, CTHREADS, smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return per > 0 ? (uint32_t)sms : 0u;
+}
+static uint32_t grid_blocks(int device, uint32_t es) {
+  static std::once_flag once[64];
+  static uint32_t blocks[64] = {};
+  if (device < 0 || device >= 64 || (es != 1 && es != 2 && es != 4)) return 0;
+  std::call_once(once[device], [device]() {
+    blocks[device] = std::min({grid_setup_es<1>(device), grid_setup_es<2>(device), grid_setup_es<4>(device)});
+  });
+  return blocks[device];
+}
+template <int ES>
+static cudaError_t launch_rounds_es(P p, bool grid, uint32_t blocks, uint32_t fs, uint32_t max_rounds,
+                                    cudaStream_t S) {
+  if (!grid) return launch_cluster_es<ES>(p, blocks, fs, max_rounds, S);
+  void *args[3] = {&p, &fs, &max_rounds};
+  return cudaLaunchCooperativeKernel((void *)k_wide_rounds<ES, true>, dim3(blocks), dim3(CTHREADS), args,
+                                     sizeof(SWarp<ES>) * CWARPS, S);
+}
+// Games of up to so many positions run their rounds in launches of one cluster,
+// of up to so many in cooperative launches.  Median per call on one B200, all
+// rounds in cluster launches / in cooperative ones:
+//   conf {30, 3}, 300 / 2,000 / 4,000 / 12,000 positions
+//     0.42 / 4.15 / 2.15 / 6.30 ms against 0.50 / 4.30 / 2.25 / 6.09;
+//   {16, 7}, 2,000 / 20,000 positions 1.37 / 3.41 against 1.47 / 2.88 ms;
+//   {1, u32::MAX}, 2,000 / 20,000 positions 0.60 / 1.75 against 0.70 / 1.58 ms.
+// Rounds as kernels with read-backs against cooperative launches: {16, 7},
+// 100,000 positions 10.2-10.9 against 8.4 ms, {1, u32::MAX}, 150,000 positions
+// 8.5 against 7.1 ms.  Warps per block: 8, 16 and 24 warps of a cluster took
+// 8.6, 8.1 and 8.6 ms for the 12,000 positions (when every supremum was
+// inserted).
+constexpr uint32_t WIDE_CLUSTER_POSITIONS = 8192, WIDE_GRID_POSITIONS = 262144;
+constexpr uint32_t WIDE_CLUSTER_ROUNDS = 256;  // per launch
 
 static geq_status check_game(const GameInput &gi, const Conf &c) {
   const geq_game_graph &g = gi.g;
@@ -1139,7 +1182,8 @@ static geq_status solve_one_game(Engine &eng, int device, const GameInput &gi, c
   p.front = d_front;
   p.next = d_next;
   uint64_t rounds = 0;
-  const uint32_t cluster = n <= WIDE_CLUSTER_POSITIONS ? cluster_blocks(device, es) : 0u;
+  const bool grid = n > WIDE_CLUSTER_POSITIONS && n <= WIDE_GRID_POSITIONS && grid_blocks(device, es) != 0u;
+  const uint32_t cluster = grid ? grid_blocks(device, es) : n <= WIDE_GRID_POSITIONS ? cluster_blocks(device, es) : 0u;
   const auto t_start = std::chrono::steady_clock::now();
   while (fsize) {
     bool first_try = true;  // of this round's slots
@@ -1147,9 +1191,9 @@ static geq_status solve_one_game(Engine &eng, int device, const GameInput &gi, c
       // rounds in one launch; a round it left unfinished goes on below
       WCU(cudaMemsetAsync(&d_ctr->next_slot, 0, 12, S));  // next_slot, n_ovf, arena_full
       p.slots = nullptr;
-      WCU(es == 1   ? launch_cluster_es<1>(p, cluster, fsize, WIDE_CLUSTER_ROUNDS, S)
-          : es == 2 ? launch_cluster_es<2>(p, cluster, fsize, WIDE_CLUSTER_ROUNDS, S)
-                    : launch_cluster_es<4>(p, cluster, fsize, WIDE_CLUSTER_ROUNDS, S));
+      WCU(es == 1   ? launch_rounds_es<1>(p, grid, cluster, fsize, WIDE_CLUSTER_ROUNDS, S)
+          : es == 2 ? launch_rounds_es<2>(p, grid, cluster, fsize, WIDE_CLUSTER_ROUNDS, S)
+                    : launch_rounds_es<4>(p, grid, cluster, fsize, WIDE_CLUSTER_ROUNDS, S));
       launches++;
       WCU(cudaMemcpyAsync(&h, d_ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, S));
       WCU(cudaStreamSynchronize(S));

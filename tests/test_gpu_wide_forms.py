@@ -1,7 +1,8 @@
 """The forms of the multi-word solver's rounds against the oracle: antichains
 in shared memory (energies of one, two and four words) up to, at and beyond
 their 256 members, other energy sizes in the warps' scratch, games whose rounds
-run inside one launch (up to 65,536 positions) and larger ones."""
+run inside launches of a cluster (up to 8,192 positions) or of the whole device
+(up to 262,144) and larger ones."""
 from __future__ import annotations
 
 import ctypes as C
@@ -102,7 +103,7 @@ def test_antichain_sizes(geq, ctx, conf, members):
 
 
 @pytest.mark.parametrize("conf", [(30, 3), (1, 0xFFFFFFFF)])
-@pytest.mark.parametrize("n", [1, 33, 65536, 65537])
+@pytest.mark.parametrize("n", [1, 33, 8192, 8193, 65536, 65537, 262144, 262145])
 def test_game_sizes(geq, ctx, conf, n):
     rng = np.random.default_rng(n)
     att = (rng.random(n) < 0.6).astype(np.uint8)
