@@ -429,6 +429,7 @@ __device__ __forceinline__ bool insert32(const P &p, uint32_t *M, uint8_t *fl, u
     if (j != lane && leq_es<ES>(xj, x, p.sw) && (j < lane || !eq_es<ES>(xj, x))) live = false;
   }
   lm = __ballot_sync(FULL, live);
+  __syncwarp();  // flags set above are read by other lanes; ballots order no memory
   if (!lm) return true;
   uint32_t rm = 0;  // bit k: member 32k + lane leaves
   for (uint32_t r = lm; r; r &= r - 1u) {
