@@ -5024,9 +5024,11 @@ geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &han
   const unsigned long long room = 4 * N + 256;  // energies the kernel writes to the host by itself
   if (!sol.off_buf.alloc(s.hpool, (N + 1) * 8)) return fail(GEQ_ERR_OUT_OF_MEMORY, "host memory for offsets");
   if (!sol.data_buf.alloc(s.hpool, room * 4)) return fail(GEQ_ERR_OUT_OF_MEMORY, "host memory for %llu words", room);
-  sa.h_in = (const uint4 *)H;
-  sa.dst = (uint4 *)base;
-  sa.in_vecs = L.rrow / sizeof(uint4);
+  // (from the row offsets on: the control block in front of them is written by
+  // one thread of the kernel while the others copy)
+  sa.h_in = (const uint4 *)(H + L.row);
+  sa.dst = (uint4 *)(base + L.row);
+  sa.in_vecs = (L.rrow - L.row) / sizeof(uint4);
   sa.h_ctr = s.h_ctr;
   // (a block from the heap, when no page-locked one could be had, is not the device's to write)
   sa.h_off = sol.off_buf.pool ? (unsigned long long *)sol.off_buf.p : nullptr;
