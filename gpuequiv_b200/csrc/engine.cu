@@ -115,9 +115,10 @@ struct Ctr {
   uint32_t next_slot;  // k_round: next frontier slot to hand out (32 per grab)
   uint32_t nbig;       // large positions queued by k_round for k_round_big
   uint32_t next_big;   // k_round_big: next queue entry to hand out
+  // (group_rounds counts the large positions of odd and even rounds in them)
   uint32_t npush;      // parts of long predecessor lists queued for k_round_big
   uint32_t next_push;  // k_round_big: next of them to hand out
-  uint32_t pad3;
+  uint32_t heavy;      // k_rounds_cluster left because of the round's large positions
   unsigned long long positions, edges, bytes, rounds;
 #if GEQ_PATH_PROFILE
   unsigned long long prof[32];
@@ -2667,6 +2668,14 @@ struct BeginArgs {
 // - larger ones, up to CLUSTER_POSITIONS_TAIL (every block counts the whole
 //   bitmap, 128 KB there), from the step on that leaves at most
 //   CLUSTER_FRONTIER positions (1,024 to 4,096: the same within noise);
+// - both only with few enough edges, and until a round has more than
+//   CLUSTER_BIG positions beyond the lane path's limits: those take a warp
+//   each, of which a cluster has 256 and k_round_big's grid 4,736.  20,000
+//   positions with 400,000 edges 27.5 -> 13.3 ms, 30,000 with 4 million 148 ->
+//   28.6 ms, 2,000 of 12,000 positions a round with lists of 20 to 110 energies
+//   2.6 -> 1.4 ms.  The line of CLUSTER_BIG at 512 / 1,024 / 1,792: 20,000
+//   positions with 120,000 edges 5.2 / 4.0 / 4.1 ms (a lone game starts again
+//   elsewhere), 8,000 with 120,000 4.7 / 4.7 / 4.0;
 // - a lone game of up to SMALL_GAME_POSITIONS is one launch from input to
 //   result: 2,500 positions 578 -> 162 us (one block of 8 warps before),
 //   9,000: 736 -> 280 us, 30,000: 720 -> 663 us (upload and graphs of rounds
@@ -2676,6 +2685,8 @@ struct BeginArgs {
 //   124), of 8 warps up to STATIC_FEW_WARPS (80 positions: 66 us, 74 with 16).
 constexpr unsigned long long CLUSTER_POSITIONS = 32768, CLUSTER_POSITIONS_TAIL = 1ull << 20;
 constexpr uint32_t CLUSTER_FRONTIER = 2048;
+constexpr unsigned long long CLUSTER_EDGES = 196608, CLUSTER_TAIL_DEGREE = TD;
+constexpr uint32_t CLUSTER_BIG = 1792;
 constexpr uint32_t CLUSTER_ROUNDS = 256, CLUSTER_ROUNDS_SERVING = 16;  // per launch
 constexpr unsigned long long STATIC_ONE_BLOCK = 400, STATIC_FEW_WARPS = 256;
 
@@ -2738,6 +2749,7 @@ struct DeviceGamesImpl {
   struct Progress {
     unsigned long long launches = 0, compactions = 0, round_launches = 0;
     double round_ms = 0.0;
+    bool heavy = false;  // rounds with many large positions: no more cluster launches
     std::chrono::steady_clock::time_point t_start{};
   } prog;
   uint32_t frontier = ~0u;  // its size after the last step (unknown before the first)
@@ -3788,13 +3800,14 @@ geq_status Engine::step_enqueue(DeviceGamesImpl &dg, bool active) {
   if (!dg.hstep.p && !dg.hstep.alloc(s.hpool, hbytes)) return fail(GEQ_ERR_OUT_OF_MEMORY, "step read-back");
   // small uploads, and the rounds of medium ones whose frontier has become
   // small, run inside one launch of a cluster of blocks
-  const bool whole = dg.N <= CLUSTER_POSITIONS;
-  if (dg.begin_pending && !(use_graph && whole)) {  // the tuning changed since solve_begin
+  const bool whole = dg.N <= CLUSTER_POSITIONS && dg.M <= CLUSTER_EDGES && !pr.heavy;
+  if (dg.begin_pending && !(use_graph && whole)) {  // the tuning changed since solve_begin, or too many edges
     dg.begin_pending = false;
     geq_status g = begin_launches(dg);
     if (g) return g;
   }
-  const bool cluster = use_graph && (whole || (dg.N <= CLUSTER_POSITIONS_TAIL && dg.frontier <= CLUSTER_FRONTIER));
+  const bool cluster = use_graph && (whole || (dg.N <= CLUSTER_POSITIONS_TAIL && dg.M <= CLUSTER_TAIL_DEGREE * dg.N &&
+                                               dg.frontier <= CLUSTER_FRONTIER && !pr.heavy));
   if (cluster) {
     BeginArgs begin{};
     if (dg.begin_pending) {
@@ -3855,6 +3868,7 @@ geq_status Engine::step_finish(DeviceGamesImpl &dg, bool &done, const uint8_t *&
     if (c.overflow) return GEQ_OK;  // the halted rounds run at the next step; nothing retires now
   }
   dg.frontier = c.fsize[c.cur];
+  pr.heavy |= c.heavy != 0u;
   if (c.fsize[c.cur] == 0) {
     done = true;
     dg.next_stamp = c.stamp + 2u;
@@ -4262,6 +4276,7 @@ struct StaticArgs {
   const uint32_t *reach;        // explicit to_reach list, or null: standard reach
   uint32_t n_reach;
   uint32_t max_rounds;
+  uint32_t max_big;  // large positions of a round beyond which the game is left to the general path
   uint32_t *arena;
   unsigned long long arena_cap;  // words
   unsigned long long *out_off;   // n_nodes + 1 result offsets
@@ -4279,9 +4294,12 @@ struct StaticArgs {
   unsigned long long h_cap;
 };
 // Games up to these sizes take the one-launch path in geq_energy_game_run.
-constexpr unsigned long long SMALL_GAME_POSITIONS = 32768, SMALL_GAME_EDGES = 8 * SMALL_GAME_POSITIONS;
+constexpr unsigned long long SMALL_GAME_POSITIONS = 32768, SMALL_GAME_EDGES = CLUSTER_EDGES;
+// Of them, games beyond these are left to the general path when a round has
+// more than CLUSTER_BIG large positions.
+constexpr unsigned long long ONE_BLOCK_POSITIONS = 4096, ONE_BLOCK_EDGES = 65536;
 // Ctr::pad bits of the static solve
-constexpr uint32_t SERR_COL = 1u, SERR_WEIGHT = 2u, SERR_ARENA = 4u, SERR_ROUNDS = 8u;
+constexpr uint32_t SERR_COL = 1u, SERR_WEIGHT = 2u, SERR_ARENA = 4u, SERR_ROUNDS = 8u, SERR_HEAVY = 16u;
 
 // ---- rounds inside one launch ------------------------------------------------
 // A cluster of blocks (or one block) that runs rounds without leaving the
@@ -4362,9 +4380,13 @@ __device__ __forceinline__ uint32_t group_fill(const KParams &p, Ctr *c, const G
 // the warp that met them), then, behind a barrier, the new descriptors
 // published, the bitmap half of the round after next cleared and the next
 // list written.
+//
+// Also left after a round with more than `max_big` large positions (returns
+// true): they take a warp each, and the cluster has 256 warps on 16 of the
+// SMs.
 template <class Cd>
-__device__ void group_rounds(const KParams &p, Ctr *c, const Group &g, RoundState &st, uint32_t max_rounds,
-                             uint32_t limit, uint32_t *dsm, uint32_t *wsum, uint32_t *flags) {
+__device__ bool group_rounds(const KParams &p, Ctr *c, const Group &g, RoundState &st, uint32_t max_rounds,
+                             uint32_t limit, uint32_t max_big, uint32_t *dsm, uint32_t *wsum, uint32_t *flags) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   uint32_t *sm = dsm + warp * CWARP_WORDS;
   uint32_t *scr = sm + W_WORDS + lane;
@@ -4376,6 +4398,7 @@ __device__ void group_rounds(const KParams &p, Ctr *c, const Group &g, RoundStat
   uint32_t t_edges = 0, t_bytes = 0, t_pos = 0;
   WarpCtx x{p, c, arena, cap, lane, sm, wa, w_edges, w_bytes, scr};
   const uint32_t warps = g.blocks * nw, gw = warp * g.blocks + g.rank;  // neighbours on different SMs
+  uint32_t left = 0;
   for (uint32_t r = 0; r < max_rounds && st.fs != 0u && st.fs <= limit; r++) {
     const uint32_t *F = st.cur ? p.front1 : p.front0;
     const uint32_t stamp = st.stamp + 1u;
@@ -4411,6 +4434,7 @@ __device__ void group_rounds(const KParams &p, Ctr *c, const Group &g, RoundStat
       if (active && ts != T_BIG && CHECK_IDX(c, slot, p.n_nodes)) p.slot_new[slot] = (ts == T_CHANGED) ? nd : NONE_DESC;
       bool retry = ts == T_OVERFLOW, changed = ts == T_CHANGED;
       uint32_t big = __ballot_sync(FULL, ts == T_BIG);
+      if (big && lane == 0) atomicAdd(st.rounds & 1u ? &c->next_big : &c->nbig, (uint32_t)__popc(big));
       while (big) {
         const uint32_t l = __ffs(big) - 1u;
         big &= big - 1u;
@@ -4447,13 +4471,17 @@ __device__ void group_rounds(const KParams &p, Ctr *c, const Group &g, RoundStat
         if (CHECK_IDX(c, v, p.n_nodes)) p.desc[v] = d;
       }
     }
-    if (threadIdx.x == 0) *flags = *(volatile uint32_t *)&c->overflow | *(volatile uint32_t *)&c->error;
+    if (threadIdx.x == 0)
+      *flags = ((*(volatile uint32_t *)&c->overflow | *(volatile uint32_t *)&c->error) ? 1u : 0u) |
+               (*(volatile uint32_t *)(st.rounds & 1u ? &c->next_big : &c->nbig) > max_big ? 2u : 0u);
+    if (g.tid == 0) *(st.rounds & 1u ? &c->nbig : &c->next_big) = 0u;  // the last round's: everyone has read it
     st.fs = group_fill(p, c, g, stamp, st.cur ? p.front0 : p.front1, wsum);  // its barriers cover *flags
     st.cur ^= 1u;
     st.stamp = stamp;
     st.rounds++;
     g.sync();
-    if (*flags) break;
+    left = *flags;
+    if (left) break;
   }
   unsigned long long te = t_edges, tb = t_bytes, tp = t_pos;
 #pragma unroll
@@ -4467,6 +4495,7 @@ __device__ void group_rounds(const KParams &p, Ctr *c, const Group &g, RoundStat
     atomicAdd(&c->edges, te + w_edges);
     atomicAdd(&c->bytes, tb + w_bytes);
   }
+  return (left & 2u) != 0u;
 }
 
 // Rounds of an upload by one cluster: the state is taken from the control
@@ -4517,8 +4546,9 @@ __global__ void __launch_bounds__(CT, 1) k_rounds_cluster(const KParams p, uint3
     g.sync();  // every block has read the state
     if (idle) return;
   }
-  group_rounds<Cd>(p, c, g, st, max_rounds, limit, dsm, wsum, &s_flags);
+  const bool heavy = group_rounds<Cd>(p, c, g, st, max_rounds, limit, CLUSTER_BIG, dsm, wsum, &s_flags);
   if (g.tid == 0) {
+    if (heavy) c->heavy = 1u;
     c->fsize[0] = st.cur ? 0u : st.fs;
     c->fsize[1] = st.cur ? st.fs : 0u;
     c->cur = st.cur;
@@ -4720,11 +4750,11 @@ __global__ void __launch_bounds__(CT, 1) k_solve_static(const KParams p, const S
   RoundState st{0u, 0u, 1u, 0u};
   st.fs = group_fill(p, c, g, st.stamp, p.front0, wsum);
   g.sync();
-  group_rounds<Cd>(p, c, g, st, a.max_rounds, ~0u, dsm, wsum, &s_flags);
+  const bool heavy = group_rounds<Cd>(p, c, g, st, a.max_rounds, ~0u, a.max_big, dsm, wsum, &s_flags);
   g.sync();
   if (g.tid == 0) {
     c->rounds = st.rounds;
-    c->pad = c->overflow ? SERR_ARENA : (!c->error && st.fs) ? SERR_ROUNDS : 0u;
+    c->pad = c->overflow ? SERR_ARENA : (c->error || !st.fs) ? 0u : heavy ? SERR_HEAVY : SERR_ROUNDS;
   }
   g.sync();
   if (c->pad || c->error) {
@@ -4905,6 +4935,7 @@ static void block_params(const BlockLayout &L, unsigned char *base, size_t bytes
   sa.reach = explicit_reach ? (const uint32_t *)(base + L.reach) : nullptr;
   sa.n_reach = explicit_reach ? n_reach : 0u;
   sa.max_rounds = 1u << 20;
+  sa.max_big = ~0u;
   sa.arena = (uint32_t *)(base + L.top);
   sa.arena_cap = (bytes - L.top) / 4;
   sa.out_off = (unsigned long long *)(base + L.out);
@@ -5029,6 +5060,7 @@ geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &han
   sa.h_in = (const uint4 *)(H + L.row);
   sa.dst = (uint4 *)(base + L.row);
   sa.in_vecs = (L.rrow - L.row) / sizeof(uint4);
+  if (N > ONE_BLOCK_POSITIONS || M > ONE_BLOCK_EDGES) sa.max_big = CLUSTER_BIG;
   sa.h_ctr = s.h_ctr;
   // (a block from the heap, when no page-locked one could be had, is not the device's to write)
   sa.h_off = sol.off_buf.pool ? (unsigned long long *)sol.off_buf.p : nullptr;
@@ -5039,10 +5071,10 @@ geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &han
   CU(cudaEventRecord(s.ev1, S));
   CU(cudaStreamSynchronize(S));
   const Ctr h = *s.h_ctr;
-  if ((h.pad & SERR_ARENA) || (h.error & ~DERR_BOUNDS)) {
+  if ((h.pad & (SERR_ARENA | SERR_HEAVY)) || (h.error & ~DERR_BOUNDS)) {
     sol.off_buf.reset();
     sol.data_buf.reset();
-    return GEQ_OK;  // the general path grows its arena
+    return GEQ_OK;  // the general path grows its arena and has every SM
   }
   handled = true;
   if (h.pad & SERR_COL) return fail(GEQ_ERR_INVALID_INPUT, "Node index too high: a successor index is out of range");

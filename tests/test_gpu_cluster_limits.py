@@ -1,0 +1,96 @@
+"""Where rounds leave the launches of one cluster (16 of the SMs) for kernels
+over the whole device: games with many edges, and rounds with more than 1,792
+positions that take a warp each."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from helpers import canon
+from oracle import ora
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def geq():
+    import gpuequiv_b200 as geq
+    return geq
+
+
+@pytest.fixture(scope="module")
+def ctx(geq):
+    c = geq.Context(0)
+    yield c
+    c.close()
+
+
+def dense_game(n, m, seed=1):
+    """Exactly m edges: a tenth of the defenders have no successors, the others
+    one to three; the attackers have the rest."""
+    rng = np.random.default_rng(seed)
+    att = (np.arange(n) % 5 < 3).astype(np.uint8)
+    A, D = np.nonzero(att)[0], np.nonzero(att == 0)[0]
+    few = np.repeat(D[len(D) // 10:], rng.integers(1, 4, len(D) - len(D) // 10))
+    src = np.sort(np.concatenate([few, A[rng.integers(0, len(A), m - len(few))]]))
+    row = np.zeros(n + 1, np.uint32)
+    np.cumsum(np.bincount(src, minlength=n), out=row[1:])
+    col = np.where(att[src] == 1, D[rng.integers(0, len(D), m)], A[rng.integers(0, len(A), m)]).astype(np.uint32)
+    wt = np.where(rng.random(m) < 0.3, np.uint32(1) << (4 * rng.integers(0, 6, m)).astype(np.uint32), 0)
+    return row, col, wt.astype(np.uint32), att
+
+
+def layers(width, depth):
+    """Attackers of layer k reach layer k-1 by a decrement of each element, so
+    all of a layer have the same list: 1, 6, 21, 56, 96, ... energies."""
+    n = width * (depth + 1)
+    att = np.ones(n, np.uint8)
+    att[:width] = 0
+    deg = np.full(n, 6)
+    deg[:width] = 0
+    row = np.zeros(n + 1, np.uint32)
+    np.cumsum(deg, out=row[1:])
+    rng = np.random.default_rng(5)
+    col = np.repeat(np.arange(depth) * width, width * 6) + rng.integers(0, width, width * depth * 6)
+    wt = np.tile(np.uint32(1) << (4 * np.arange(6)).astype(np.uint32), width * depth)
+    return row, col.astype(np.uint32), wt.astype(np.uint32), att
+
+
+def solve(geq, ctx, g, form):
+    graphs = [geq.GameGraph.from_csr(*g, geq.EnergyConf.STANDARD)]
+    if form == "batch":
+        graphs.append(geq.GameGraph.empty(geq.EnergyConf.STANDARD))
+    offs, data, stats = geq.run_batch_raw(graphs, ctx)
+    return offs[0].astype(np.int64), data[0], stats
+
+
+@pytest.mark.parametrize("form", ["run", "batch"])
+@pytest.mark.parametrize("n,m", [(2500, 196608), (2500, 196609), (9000, 196608), (9000, 196609), (700, 300000)])
+def test_edges(geq, ctx, n, m, form):
+    g = dense_game(n, m)
+    o, d, stats = solve(geq, ctx, g, form)
+    if m > 196608:  # every round by the four kernels
+        assert stats["kernel_launches"] >= 4 * stats["rounds"]
+    exp = ora.run_game(6, 3, *g, ora.standard_reach(g[0], g[3])).lists()
+    for v in range(n):
+        assert canon(d[o[v]:o[v + 1]]) == canon(exp[v]), f"position {v}"
+
+
+@pytest.mark.parametrize("form", ["run", "batch"])
+@pytest.mark.parametrize("width", [1792, 1793, 3000])
+def test_large_positions(geq, ctx, width, form):
+    """Layers of `width` positions whose lists leave the lane path from the
+    second layer on."""
+    depth = 6
+    g = layers(width, depth)
+    o, d, stats = solve(geq, ctx, g, form)
+    if width > 1792:
+        assert stats["kernel_launches"] >= 4 * (depth - 3)
+    g1 = layers(1, depth)
+    exp = ora.run_game(6, 3, *g1, ora.standard_reach(g1[0], g1[3])).lists()
+    for k in range(depth + 1):
+        want = np.sort(np.asarray(exp[k]).reshape(-1)).astype(np.uint32)
+        lens = np.diff(o)[k * width:(k + 1) * width]
+        assert (lens == len(want)).all(), f"layer {k}"
+        got = np.sort(d[o[k * width]:o[(k + 1) * width]].reshape(width, len(want)), axis=1)
+        assert (got == want).all(), f"layer {k}"
