@@ -2682,13 +2682,15 @@ struct BeginArgs {
 //   before);
 // - of those, up to STATIC_ONE_BLOCK by one block, whose barrier is cheaper
 //   than a cluster's (300 positions: 105 against 126 us; 800: 129 against
-//   124), of 8 warps up to STATIC_FEW_WARPS (80 positions: 66 us, 74 with 16).
+//   124), of 8 warps up to STATIC_FEW_WARPS (80 positions: 66 us, 74 with 16),
+//   while their edges are few: 400 positions with 10,000 edges 2.9 ms in one
+//   block, 1.4 in a cluster, with 160,000 7.2 and 2.5 ms.
 constexpr unsigned long long CLUSTER_POSITIONS = 32768, CLUSTER_POSITIONS_TAIL = 1ull << 20;
 constexpr uint32_t CLUSTER_FRONTIER = 2048;
 constexpr unsigned long long CLUSTER_EDGES = 196608, CLUSTER_TAIL_DEGREE = TD;
 constexpr uint32_t CLUSTER_BIG = 1792;
 constexpr uint32_t CLUSTER_ROUNDS = 256, CLUSTER_ROUNDS_SERVING = 16;  // per launch
-constexpr unsigned long long STATIC_ONE_BLOCK = 400, STATIC_FEW_WARPS = 256;
+constexpr unsigned long long STATIC_ONE_BLOCK = 400, STATIC_FEW_WARPS = 256, STATIC_ONE_BLOCK_EDGES = 4096;
 
 struct Engine::State {
   cudaStream_t stream = nullptr;
@@ -4849,7 +4851,7 @@ static geq_status launch_finish_cluster(const Engine &E, const FinishArgs &a, bo
 }
 static geq_status launch_solve_static(const KParams &kp, const StaticArgs &sa, bool generic, uint32_t blocks,
                                       cudaStream_t S) {
-  if (kp.n_nodes <= STATIC_ONE_BLOCK) blocks = 1;
+  if (kp.n_nodes <= STATIC_ONE_BLOCK && kp.n_edges <= STATIC_ONE_BLOCK_EDGES) blocks = 1;
   const uint32_t warps = blocks == 1 && kp.n_nodes <= STATIC_FEW_WARPS ? 8u : CW;
   CU(generic ? launch_cluster(k_solve_static<CodecGen>, blocks, warps, S, kp, sa)
              : launch_cluster(k_solve_static<CodecStd>, blocks, warps, S, kp, sa));

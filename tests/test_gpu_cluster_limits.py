@@ -3,6 +3,8 @@ over the whole device: games with many edges, and rounds with more than 1,792
 positions that take a warp each."""
 from __future__ import annotations
 
+import time
+
 import numpy as np
 import pytest
 
@@ -56,6 +58,12 @@ def layers(width, depth):
     return row, col.astype(np.uint32), wt.astype(np.uint32), att
 
 
+def seconds(call):
+    t0 = time.perf_counter()
+    call()
+    return time.perf_counter() - t0
+
+
 def solve(geq, ctx, g, form):
     graphs = [geq.GameGraph.from_csr(*g, geq.EnergyConf.STANDARD)]
     if form == "batch":
@@ -94,3 +102,18 @@ def test_large_positions(geq, ctx, width, form):
         assert (lens == len(want)).all(), f"layer {k}"
         got = np.sort(d[o[k * width]:o[(k + 1) * width]].reshape(width, len(want)), axis=1)
         assert (got == want).all(), f"layer {k}"
+
+
+@pytest.mark.parametrize("m", [4096, 4097, 65536, 160000])
+def test_few_positions_many_edges(geq, ctx, m):
+    """400 positions in one block up to 4,096 edges, in a cluster above; alone
+    a game is not slower than beside an empty one (an upload and its rounds)."""
+    g = dense_game(400, m, seed=3)
+    o, d, _ = solve(geq, ctx, g, "run")
+    exp = ora.run_game(6, 3, *g, ora.standard_reach(g[0], g[3])).lists()
+    for v in range(400):
+        assert canon(d[o[v]:o[v + 1]]) == canon(exp[v]), f"position {v}"
+    if m > 65536:  # whole calls: a game alone is uploaded inside its launch
+        alone = min(seconds(lambda: solve(geq, ctx, g, "run")) for _ in range(5))
+        beside = min(seconds(lambda: solve(geq, ctx, g, "batch")) for _ in range(5))
+        assert alone < 1.5 * beside, (alone, beside)
