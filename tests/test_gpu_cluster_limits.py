@@ -117,3 +117,45 @@ def test_few_positions_many_edges(geq, ctx, m):
         alone = min(seconds(lambda: solve(geq, ctx, g, "run")) for _ in range(5))
         beside = min(seconds(lambda: solve(geq, ctx, g, "batch")) for _ in range(5))
         assert alone < 1.5 * beside, (alone, beside)
+
+
+@pytest.mark.parametrize("n,width", [(3000, 1), (3000, 16), (3000, 17), (20000, 1), (20000, 16)])
+def test_rounds_of_few_positions(geq, ctx, n, width):
+    """Chains side by side, joined at their ends: rounds of `width` positions,
+    which block 0 runs alone up to 16, between wider ones."""
+    k = n // width
+    at = np.arange(k * width).reshape(width, k)  # chain j: at[j, 0] (a sink) <- at[j, 1] <- ...
+    att = np.tile((np.arange(k) % 3 != 0).astype(np.uint8), width)
+    src = [at[:, 1:].reshape(-1)]
+    dst = [at[:, :-1].reshape(-1)]
+    # a fan of 40 attackers over the chains' ends and of 40 more over those
+    fan = k * width + np.arange(80)
+    src += [np.repeat(fan[:40], width), np.repeat(fan[40:], 2)]
+    dst += [np.tile(at[:, -1], 40), fan[:40][(np.arange(80) * 7) % 40]]
+    att = np.append(att, np.ones(80, np.uint8))
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    order = np.argsort(src, kind="stable")
+    src, dst = src[order], dst[order].astype(np.uint32)
+    row = np.zeros(len(att) + 1, np.uint32)
+    np.cumsum(np.bincount(src, minlength=len(att)), out=row[1:])
+    rng = np.random.default_rng(n + width)
+    wt = np.where(rng.random(len(src)) < 0.01, np.uint32(1) << (4 * rng.integers(0, 6, len(src))).astype(np.uint32), 0)
+    g = (row, dst, wt.astype(np.uint32), att)
+    exp = ora.run_game(6, 3, *g, ora.standard_reach(row, att)).lists()
+    for form in ("run", "batch"):
+        o, d, stats = solve(geq, ctx, g, form)
+        assert stats["rounds"] >= k
+        for v in range(len(att)):
+            assert canon(d[o[v]:o[v + 1]]) == canon(exp[v]), f"position {v}"
+
+
+def test_chain_time(geq, ctx):
+    """A chain alone (a cluster) against the call that is always one block."""
+    n = 4000
+    row = np.minimum(np.arange(n + 1), n - 1).astype(np.uint32)
+    att = np.tile(np.array([1, 0], np.uint8), n // 2)
+    g = geq.GameGraph.from_csr(row, np.arange(1, n, dtype=np.uint32), np.zeros(n - 1, np.uint32), att,
+                               geq.EnergyConf.STANDARD)
+    alone = min(seconds(lambda: geq.run_batch_raw([g], ctx)) for _ in range(5))
+    block = min(seconds(lambda: geq.run_static(g, ctx)) for _ in range(5))
+    assert alone < 1.25 * block, (alone, block)
