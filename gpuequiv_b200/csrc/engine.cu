@@ -4514,8 +4514,10 @@ __device__ bool group_rounds(const KParams &p, Ctr *c, const Group &g, RoundStat
       h.sync();
       if (g.tid == 0) c->npush = 0u;  // the next round's warps add to it behind the barrier below
     }
+    // (what every block reads alike: an index a checked build refuses may be
+    // found behind the barrier, and then ends the solve when the rounds do)
     if (threadIdx.x == 0)
-      *flags = ((*(volatile uint32_t *)&c->overflow | *(volatile uint32_t *)&c->error) ? 1u : 0u) |
+      *flags = ((*(volatile uint32_t *)&c->overflow | (*(volatile uint32_t *)&c->error & ~DERR_BOUNDS)) ? 1u : 0u) |
                (*(volatile uint32_t *)(st.rounds & 1u ? &c->next_big : &c->nbig) > max_big ? 2u : 0u);
     if (g.tid == 0) *(st.rounds & 1u ? &c->nbig : &c->next_big) = 0u;  // the last round's: everyone has read it
     st.fs = group_fill(p, c, h, per, stamp, st.cur ? p.front0 : p.front1, wsum);  // its barriers cover *flags
