@@ -4300,8 +4300,10 @@ struct StaticArgs {
 // Games up to these sizes take the one-launch path in geq_energy_game_run.
 constexpr unsigned long long SMALL_GAME_POSITIONS = 32768, SMALL_GAME_EDGES = CLUSTER_EDGES;
 // Of them, games beyond these are left to the general path when a round has
-// more than CLUSTER_BIG large positions.
+// more than CLUSTER_BIG large positions, and after LARGE_ROUNDS rounds (a round
+// is 5 to 20 us): it looks at the time limit between its steps.
 constexpr unsigned long long ONE_BLOCK_POSITIONS = 4096, ONE_BLOCK_EDGES = 65536;
+constexpr uint32_t LARGE_ROUNDS = 4096;
 // Ctr::pad bits of the static solve
 constexpr uint32_t SERR_COL = 1u, SERR_WEIGHT = 2u, SERR_ARENA = 4u, SERR_ROUNDS = 8u, SERR_HEAVY = 16u;
 
@@ -5104,7 +5106,11 @@ geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &han
   sa.h_in = (const uint4 *)(H + L.row);
   sa.dst = (uint4 *)(base + L.row);
   sa.in_vecs = (L.rrow - L.row) / sizeof(uint4);
-  if (N > ONE_BLOCK_POSITIONS || M > ONE_BLOCK_EDGES) sa.max_big = CLUSTER_BIG;
+  const bool large = N > ONE_BLOCK_POSITIONS || M > ONE_BLOCK_EDGES;
+  if (large) {
+    sa.max_big = CLUSTER_BIG;
+    sa.max_rounds = LARGE_ROUNDS;
+  }
   sa.h_ctr = s.h_ctr;
   // (a block from the heap, when no page-locked one could be had, is not the device's to write)
   sa.h_off = sol.off_buf.pool ? (unsigned long long *)sol.off_buf.p : nullptr;
@@ -5115,10 +5121,10 @@ geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &han
   CU(cudaEventRecord(s.ev1, S));
   CU(cudaStreamSynchronize(S));
   const Ctr h = *s.h_ctr;
-  if ((h.pad & (SERR_ARENA | SERR_HEAVY)) || (h.error & ~DERR_BOUNDS)) {
+  if ((h.pad & (SERR_ARENA | SERR_HEAVY)) || (large && (h.pad & SERR_ROUNDS)) || (h.error & ~DERR_BOUNDS)) {
     sol.off_buf.reset();
     sol.data_buf.reset();
-    return GEQ_OK;  // the general path grows its arena and has every SM
+    return GEQ_OK;  // the general path grows its arena, has every SM and a time limit
   }
   handled = true;
   if (h.pad & SERR_COL) return fail(GEQ_ERR_INVALID_INPUT, "Node index too high: a successor index is out of range");

@@ -1,0 +1,34 @@
+"""Games of very many rounds: the time limit between steps holds for lone games
+of every size above 4,096 positions, and in the server they do not hold up
+other requests."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def chain(geq, n):
+    row = np.minimum(np.arange(n + 1), n - 1).astype(np.uint32)
+    att = (np.arange(n) % 2 != (n - 1) % 2).astype(np.uint8)  # the last position is a defender
+    return geq.GameGraph.from_csr(row, np.arange(1, n, dtype=np.uint32), np.zeros(n - 1, np.uint32), att,
+                                  geq.EnergyConf.STANDARD)
+
+
+@pytest.mark.parametrize("n", [4097, 4098, 20000, 32768, 32769])
+def test_time_limit(monkeypatch, n):
+    import gpuequiv_b200 as geq
+    ctx = geq.Context(0)
+    g = chain(geq, n)
+    offs, data, stats = geq.run_batch_raw([g], ctx)
+    assert stats["rounds"] >= n - 1
+    assert np.array_equal(offs[0], np.arange(n + 1)) and not data[0].any()
+    if n > 5000:  # (up to 4,096 rounds in one launch)
+        monkeypatch.setenv("GEQ_SOLVE_TIMEOUT_S", "0.0001")
+        with pytest.raises(geq.GeqError, match="no fixpoint"):
+            geq.run_batch_raw([g], ctx)
+        monkeypatch.delenv("GEQ_SOLVE_TIMEOUT_S")
+        offs, data, _ = geq.run_batch_raw([g], ctx)  # the context goes on
+        assert np.array_equal(offs[0], np.arange(n + 1)) and not data[0].any()
+    ctx.close()
