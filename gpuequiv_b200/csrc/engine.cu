@@ -4301,9 +4301,9 @@ struct StaticArgs {
 constexpr unsigned long long SMALL_GAME_POSITIONS = 32768, SMALL_GAME_EDGES = CLUSTER_EDGES;
 // Of them, games beyond these are left to the general path when a round has
 // more than CLUSTER_BIG large positions, and after LARGE_ROUNDS rounds (a round
-// is 5 to 20 us): it looks at the time limit between its steps.
+// is 5 to 20 us): it looks at the time limit between its steps.  (The server
+// gives them fewer rounds, or none.)
 constexpr unsigned long long ONE_BLOCK_POSITIONS = 4096, ONE_BLOCK_EDGES = 65536;
-constexpr uint32_t LARGE_ROUNDS = 4096;
 // Ctr::pad bits of the static solve
 constexpr uint32_t SERR_COL = 1u, SERR_WEIGHT = 2u, SERR_ARENA = 4u, SERR_ROUNDS = 8u, SERR_HEAVY = 16u;
 
@@ -5065,7 +5065,7 @@ geq_status Engine::run_static(int device, const geq_game_graph &g, const uint32_
 // game from page-locked staging and writes the lists to page-locked memory, so
 // the call waits once.  A game whose lists outgrow the block's arena is left to the general path
 // (handled = false), as is everything outside the limits.
-geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &handled) {
+geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &handled, uint32_t large_rounds) {
   handled = false;
   State &s = *st;
   cudaStream_t S = s.stream;
@@ -5073,6 +5073,8 @@ geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &han
   const unsigned long long N = gi.g.n_vertices, M = gi.g.row_offsets[gi.g.n_vertices];
   if (gi.init || tuning.flags || N > SMALL_GAME_POSITIONS || M > SMALL_GAME_EDGES || !conf.supported())
     return GEQ_OK;
+  const bool large = N > ONE_BLOCK_POSITIONS || M > ONE_BLOCK_EDGES;
+  if (large && !large_rounds) return GEQ_OK;
   const BlockLayout L = block_layout(N, M, gi.n_reach);
   const size_t bytes = L.top + 4 * (16 * (size_t)(N + M) + 65536);
   unsigned char *base = (unsigned char *)s.pool.get(bytes);
@@ -5106,10 +5108,9 @@ geq_status Engine::solve_small(const GameInput &gi, geq_solution &sol, bool &han
   sa.h_in = (const uint4 *)(H + L.row);
   sa.dst = (uint4 *)(base + L.row);
   sa.in_vecs = (L.rrow - L.row) / sizeof(uint4);
-  const bool large = N > ONE_BLOCK_POSITIONS || M > ONE_BLOCK_EDGES;
   if (large) {
     sa.max_big = CLUSTER_BIG;
-    sa.max_rounds = LARGE_ROUNDS;
+    sa.max_rounds = large_rounds;
   }
   sa.h_ctr = s.h_ctr;
   // (a block from the heap, when no page-locked one could be had, is not the device's to write)

@@ -249,7 +249,10 @@ class Engine {
                                const std::vector<uint32_t> &count, geq_solution &sol);
   // One small game (no initial lists, default tuning) by one launch of
   // k_solve_static in a pooled block; handled = false leaves it to upload/solve.
-  geq_status solve_small(const GameInput &gi, geq_solution &sol, bool &handled);
+  // Games above 4,096 positions or 65,536 edges get large_rounds rounds (0:
+  // they are left to upload/solve at once).
+  static constexpr uint32_t LARGE_ROUNDS = 4096;
+  geq_status solve_small(const GameInput &gi, geq_solution &sol, bool &handled, uint32_t large_rounds = LARGE_ROUNDS);
   // geq_energy_game_run_static: one game in the file-scope scratch, no allocation.
   geq_status run_static(int device, const geq_game_graph &g, const uint32_t *to_reach, uint32_t n_reach,
                         uint64_t *offsets, uint32_t *data, uint64_t data_cap, uint64_t *n_words,

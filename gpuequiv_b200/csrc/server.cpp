@@ -225,7 +225,10 @@ geq_status retire(Engine &e, Session &ss, const std::vector<uint32_t> &games, st
 // Games of one conf with a thermometer codec: a lone small game in one
 // launch (Engine::solve_small), else an upload that becomes a session.  An
 // upload of several games that fails is retried game by game, so that a
-// malformed game fails alone.
+// malformed game fails alone.  The launch of a larger lone game is taken only
+// by a pipeline without sessions and for IDLE_ROUNDS rounds (a spectroscopy game
+// of 30,000 positions has some 30, 0.7 ms): it holds up what arrives meanwhile.
+constexpr uint32_t IDLE_ROUNDS = 256;
 void start_games(Engine &e, std::vector<Request *> &batch, uint64_t footprint,
                  std::vector<std::unique_ptr<Session>> &out, std::vector<Request *> &done) {
   std::vector<GameInput> in(batch.size());
@@ -246,7 +249,7 @@ void start_games(Engine &e, std::vector<Request *> &batch, uint64_t footprint,
   if (batch.size() == 1) {
     std::unique_ptr<geq_solution> one(new geq_solution());
     bool handled = false;
-    const geq_status st = e.solve_small(in[0], *one, handled);
+    const geq_status st = e.solve_small(in[0], *one, handled, out.empty() ? IDLE_ROUNDS : 0u);
     if (st) return fail_req(batch[0], st, geq_last_error(), done);
     if (handled) {
       batch[0]->sol = std::move(one);

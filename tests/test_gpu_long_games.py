@@ -32,3 +32,26 @@ def test_time_limit(monkeypatch, n):
         offs, data, _ = geq.run_batch_raw([g], ctx)  # the context goes on
         assert np.array_equal(offs[0], np.arange(n + 1)) and not data[0].any()
     ctx.close()
+
+
+def test_server_short_beside_long():
+    """One pipeline: a chain of 32,000 rounds (some 0.2 s) and then short games,
+    lone requests all; the short ones are answered while the chain is solved."""
+    import gpuequiv_b200 as geq
+    from gpuequiv_b200.serving import Server
+    ctx = geq.Context(0)
+    long, short = chain(geq, 32000), chain(geq, 20)
+    with Server(ctx, n_pipelines=1) as srv:
+        for g in (short, long):  # everything allocated and loaded
+            srv.poll(srv.submit(g))
+        t = srv.submit(long)
+        assert srv.poll(t, 5) is None  # taken by the pipeline
+        early = 0
+        for _ in range(5):
+            got = srv.poll(srv.submit(short))
+            assert np.array_equal(got[0], np.arange(21))
+            early += srv.stats()["running"] >= 1  # the chain
+        assert early == 5
+        got = srv.poll(t)
+        assert np.array_equal(got[0], np.arange(32001)) and not got[1].any()
+    ctx.close()
