@@ -159,3 +159,21 @@ def test_chain_time(geq, ctx):
     alone = min(seconds(lambda: geq.run_batch_raw([g], ctx)) for _ in range(5))
     block = min(seconds(lambda: geq.run_static(g, ctx)) for _ in range(5))
     assert alone < 1.25 * block, (alone, block)
+
+
+def test_two_large_positions_a_round(geq, ctx):
+    """Two positions a round take as long as one: each has a warp."""
+    conf = geq.EnergyConf(8, 4)
+
+    def call(width):
+        depth = 5
+        row = np.concatenate([np.zeros(width), np.arange(width * depth + 1) * 8]).astype(np.uint32)
+        col = np.repeat(np.arange(depth * width), 8).astype(np.uint32)
+        wt = np.tile(np.uint32(1) << (4 * np.arange(8)).astype(np.uint32), width * depth).astype(np.uint32)
+        att = (np.arange(width * (depth + 1)) >= width).astype(np.uint8)
+        g = geq.GameGraph.from_csr(row, col, wt, att, conf)
+        empty = geq.GameGraph.empty(conf)
+        return [min(seconds(lambda: geq.run_batch_raw(gs, ctx)) for _ in range(4)) for gs in ([g], [g, empty])]
+
+    for one, two in zip(call(1), call(2)):
+        assert two < 1.4 * one, (one, two)
