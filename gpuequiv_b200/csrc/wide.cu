@@ -899,32 +899,53 @@ __global__ void k_wide_redesc(unsigned long long *desc, const unsigned long long
                                        "%s: %s", #x, cudaGetErrorString(e_));           \
   } while (0)
 
-// Device buffers of one solve from the engine's pool (all work is on the
-// engine's stream).  The device's stream-ordered pool gives its memory back at
-// every wait unless told otherwise: a solve's 18 buffers then cost 10 to 60 ms.
+// Device buffers of one solve (all work is on the engine's stream).  Blocks up
+// to POOL_MAX come from the engine's pool: the device's stream-ordered pool gives
+// its memory back at every wait unless told otherwise, which for a solve's 18
+// buffers cost 10 to 60 ms.  Larger ones -- arenas of big games, the warps'
+// scratch of up to 4 GB -- come from that pool and go back to the device when
+// the solve ends.  (A line of 32 MB instead: games that use the smallest
+// scratch, 155 MB, 11.5 -> 14.1 ms.)
 struct Bufs {
+  static constexpr size_t POOL_MAX = 256u << 20;
+  struct Block {
+    void *p;
+    size_t bytes;
+    bool pooled;
+  };
   Engine &eng;
-  std::vector<std::pair<void *, size_t>> ptrs;
+  std::vector<Block> blocks;
+  cudaStream_t stream() const { return (cudaStream_t)eng.stream_handle(); }
   template <class T>
   geq_status get(T *&p, size_t n) {
-    const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-    void *q = eng.pool_get(bytes);
-    if (!q) return fail(GEQ_ERR_OUT_OF_MEMORY, "device allocation of %zu bytes for the wide solver failed", bytes);
-    ptrs.emplace_back(q, bytes);
-    p = (T *)q;
+    Block b{nullptr, std::max<size_t>(n, 1) * sizeof(T), false};
+    b.pooled = b.bytes <= POOL_MAX;
+    if (!b.pooled && cudaMallocAsync(&b.p, b.bytes, stream()) != cudaSuccess) {
+      cudaGetLastError();
+      b.p = nullptr;
+      b.pooled = true;  // the engine's pool gives up its idle blocks first
+    }
+    if (b.pooled) b.p = eng.pool_get(b.bytes);
+    if (!b.p) return fail(GEQ_ERR_OUT_OF_MEMORY, "device allocation of %zu bytes for the wide solver failed", b.bytes);
+    blocks.push_back(b);
+    p = (T *)b.p;
     return GEQ_OK;
   }
+  void give(const Block &b) {
+    if (b.pooled) eng.pool_put(b.p, b.bytes);
+    else cudaFreeAsync(b.p, stream());
+  }
   void put(void *q) {
-    for (auto &x : ptrs)
-      if (x.first == q) {
-        eng.pool_put(q, x.second);
-        x.first = nullptr;
+    for (size_t i = 0; i < blocks.size(); i++)
+      if (blocks[i].p == q) {
+        give(blocks[i]);
+        blocks.erase(blocks.begin() + i);
+        return;
       }
   }
   ~Bufs() {
-    cudaStreamSynchronize((cudaStream_t)eng.stream_handle());  // error paths leave work behind
-    for (auto &x : ptrs)
-      if (x.first) eng.pool_put(x.first, x.second);
+    cudaStreamSynchronize(stream());  // error paths leave work behind
+    for (auto &b : blocks) give(b);
   }
 };
 
