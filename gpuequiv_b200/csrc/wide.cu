@@ -1204,6 +1204,7 @@ static geq_status solve_one_game(Engine &eng, int device, const GameInput &gi, c
   p.front = d_front;
   p.next = d_next;
   uint64_t rounds = 0;
+  uint32_t *d_items = nullptr;  // the slots of a round that are computed again
   const bool grid = n > WIDE_CLUSTER_POSITIONS && n <= WIDE_GRID_POSITIONS && grid_blocks(device, es) != 0u;
   const uint32_t cluster = grid ? grid_blocks(device, es) : n <= WIDE_GRID_POSITIONS ? cluster_blocks(device, es) : 0u;
   const auto t_start = std::chrono::steady_clock::now();
@@ -1296,7 +1297,7 @@ static geq_status solve_one_game(Engine &eng, int device, const GameInput &gi, c
           1, std::min<unsigned long long>(max_warps, (4ull << 30) / (scratch_words * 4)));
       if ((st = B.get(d_scratch, scratch_words * scratch_warps))) return st;
       // the overflowed slots become the items (copied: the kernel appends to ovf)
-      uint32_t *d_items;
+      if (d_items) B.put(d_items);  // (its last reader is ahead on the stream)
       if ((st = B.get(d_items, h.n_ovf))) return st;
       WCU(cudaMemcpyAsync(d_items, d_ovf, h.n_ovf * 4ull, cudaMemcpyDeviceToDevice, S));
       p.scratch = d_scratch;
