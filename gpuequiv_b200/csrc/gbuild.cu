@@ -465,7 +465,8 @@ __global__ void __launch_bounds__(GH_WARPS * 32) k_gen_heavy(View v, const unsig
 // hundred states has 5 to 30 such levels.  A cluster of blocks runs the same
 // functors phase after phase with the cluster's hardware barrier between them
 // (nothing spins), level after level, until the frontier runs empty, outgrows
-// `limit` or a buffer must grow.
+// `limit`, a buffer must grow or max_levels levels have run (a chain-shaped
+// system has as many levels as it is long).
 namespace cg = cooperative_groups;
 constexpr uint32_t CLW = 16;  // warps per block
 constexpr uint32_t CLT = 32 * CLW;
@@ -569,7 +570,8 @@ __device__ __forceinline__ void cl_scan(const Cluster &g, const uint32_t (&n)[R]
   }
 }
 
-__global__ void __launch_bounds__(CLT, 1) k_levels_cluster(View v, uint32_t start, uint32_t n_starts, uint32_t limit) {
+__global__ void __launch_bounds__(CLT, 1) k_levels_cluster(View v, uint32_t start, uint32_t n_starts, uint32_t limit,
+                                                           uint32_t max_levels) {
   extern __shared__ uint32_t bm_all[];
   __shared__ ScanSh sh;
   const Cluster g = this_cluster_threads();
@@ -622,7 +624,7 @@ __global__ void __launch_bounds__(CLT, 1) k_levels_cluster(View v, uint32_t star
   }
   if (one) v.ctl->n_heavy = 0u;
   g.sync();
-  for (;;) {
+  for (uint32_t k = 0; k < max_levels; k++) {
     const unsigned long long F = v.t[T_F];
     if (!v.t[T_GO] || F > limit) break;
     if (F == 0 || F > v.capF) {
@@ -1047,8 +1049,8 @@ struct DevBackend {
     note(cudaLaunchKernelEx(&cfg, f, args...));
     launches++;
   }
-  void cluster_levels(const View &v, bool start, uint32_t n_starts) {
-    launch_cluster(k_levels_cluster, CL_SMEM, v, start ? 1u : 0u, n_starts, CL_FRONTIER);
+  void cluster_levels(const View &v, bool start, uint32_t n_starts, uint32_t max_levels) {
+    launch_cluster(k_levels_cluster, CL_SMEM, v, start ? 1u : 0u, n_starts, CL_FRONTIER, max_levels);
   }
   // one thread per state and per job, twice over at most
   bool cluster_refine_ok(uint32_t states, uint32_t jobs) const {

@@ -781,7 +781,7 @@ struct LevelEndF {
 // A backend with `static constexpr bool kCluster = true` also runs levels with
 // small frontiers in one launch:
 //   bool cluster_ok(uint32_t items);          frontiers of that many positions go there
-//   void cluster_levels(const View &, bool start, uint32_t n_starts);   (start: the start level first)
+//   void cluster_levels(const View &, bool start, uint32_t n_starts, uint32_t max_levels);   (start: the start level first)
 //   void cluster_assemble(const View &, const Out &, uint32_t N);  jbase .. jm as after the level loop
 //   bool cluster_refine_ok(uint32_t states, uint32_t jobs); void cluster_refine(const rf::Small &);  (refine.cuh)
 //   void fetch3(h0, d0, b0, h1, d1, b1, h2, d2, b2);  three fetches and one wait
@@ -1177,8 +1177,8 @@ class Builder {
       if (!ok) return 1;
       short_ = 0;
     }
-    // levels per graph launch: the loop stops by itself when the frontier
-    // runs empty or a level stalls; the limit only bounds one launch
+    // levels per graph or cluster launch: the loop stops by itself when the
+    // frontier runs empty or a level stalls; the limit only bounds one launch
     const uint32_t batch = 4096;
     unsigned long long last_stall = ~0ull;
     uint32_t same_stall = 0;
@@ -1189,7 +1189,7 @@ class Builder {
       cluster = start;
       if constexpr (has_cluster<B>::value) {
         cluster = start || be_.cluster_ok((uint32_t)std::min<unsigned long long>(h_tot_.t[T_F], 0xffffffffull));
-        if (cluster) be_.cluster_levels(v_, start, T);
+        if (cluster) be_.cluster_levels(v_, start, T, batch);
       }
       start = false;
       if (!cluster) {

@@ -55,3 +55,26 @@ def test_server_short_beside_long():
         got = srv.poll(t)
         assert np.array_equal(got[0], np.arange(32001)) and not got[1].any()
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [2000, 50000])
+def test_levels_per_launch(n):
+    """GameBuild of two chains that differ at their ends: a level per position
+    and more, at most 4,096 levels a launch."""
+    import gpuequiv_b200 as geq
+    ctx = geq.Context(0)
+    s = np.arange(n - 1)
+    src, dst = np.concatenate([s, s + n]), np.concatenate([s + 1, s + 1 + n])
+    label = np.concatenate([np.ones(n - 1), np.ones(n - 1)]).astype(np.int32)
+    label[-1] = 2
+    lts = geq.TransitionSystem.from_arrays(src.astype(np.uint32), dst.astype(np.uint32), label, 2 * n)
+    geq.GameBatch([(lts, 0, n)], ctx)  # the next build starts with buffers of its size
+    b = geq.GameBatch([(lts, 0, n)], ctx)
+    exp = geq.GameBuild.compare(lts, 0, n).game
+    got = b.graph(0)
+    for f in ("row_offsets", "column_indices", "attacker_pos"):
+        assert np.array_equal(getattr(got, f), getattr(exp, f)), f
+    info = b.stats
+    assert info["levels"] >= n
+    assert info["kernel_launches"] >= 1 + -(-info["levels"] // 4096)  # and the assembly's
+    ctx.close()
