@@ -1166,10 +1166,8 @@ static geq_status device_build(Engine &eng, int device, uint32_t n_jobs, const L
   // freed blocks cached in this process instead of returning them at every
   // synchronisation
   static std::once_flag pool_once[64];
-  static uint32_t cluster_blocks[64] = {};
   if (device >= 0 && device < 64)
     std::call_once(pool_once[device], [device]() {
-      cluster_blocks[device] = gb::DevBackend::cluster_setup();
       cudaMemPool_t pool;
       if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
         uint64_t keep = ~0ull;
@@ -1184,7 +1182,8 @@ static geq_status device_build(Engine &eng, int device, uint32_t n_jobs, const L
   // GEQ_TUNE_NO_GRAPH: levels as plain launches (ncu does not profile the
   // kernels of a graph with conditional nodes)
   be.plain = (eng.tuning.flags & GEQ_TUNE_NO_GRAPH) != 0;
-  be.cluster_blocks = device >= 0 && device < 64 ? cluster_blocks[device] : 0u;
+  if (eng.build_cluster < 0) eng.build_cluster = (int)gb::DevBackend::cluster_setup();
+  be.cluster_blocks = (uint32_t)eng.build_cluster;
   // stage the LTSs: soff | slab | stgt | sjob | p0 | q0
   const auto t0 = clk::now();
   const size_t o_soff = 0, o_slab = o_soff + (NS + 1) * 4, o_stgt = o_slab + MS * 4, o_sjob = o_stgt + MS * 4,

@@ -266,6 +266,11 @@ class Engine {
   // Device blocks from the engine's pool, for users of the engine's stream.
   void *pool_get(size_t bytes);
   void pool_put(void *p, size_t bytes);
+  // Blocks of the device builder's cluster kernels, and of the multi-word
+  // solver's cluster and cooperative ones (0: none), set up on first use.  Per
+  // engine, not per process: the kernels' attributes belong to the CUDA
+  // context and are gone when the device was reset between two engines.
+  int build_cluster = -1, wide_cluster = -1, wide_grid = -1;
   geq_tuning tuning{};
   int n_sms = 0;
   uint64_t total_mem = 0;

@@ -949,7 +949,7 @@ struct Bufs {
   }
 };
 
-// The cluster kernels on the current device (once): blocks per cluster, 0: none.
+// The cluster kernels on the current device: blocks per cluster, 0: none.
 template <int ES>
 static uint32_t cluster_setup_es() {
   const size_t smem = sizeof(SWarp<ES>) * CWARPS;
@@ -975,14 +975,11 @@ static uint32_t cluster_setup_es() {
   }
   return 0;
 }
-static uint32_t cluster_blocks(int device, uint32_t es) {
-  static std::once_flag once[64];
-  static uint32_t blocks[64] = {};
-  if (device < 0 || device >= 64 || (es != 1 && es != 2 && es != 4)) return 0;
-  std::call_once(once[device], [device]() {
-    blocks[device] = std::min({cluster_setup_es<1>(), cluster_setup_es<2>(), cluster_setup_es<4>()});
-  });
-  return blocks[device];
+static uint32_t cluster_blocks(Engine &eng, uint32_t es) {
+  if (es != 1 && es != 2 && es != 4) return 0;
+  if (eng.wide_cluster < 0)
+    eng.wide_cluster = (int)std::min({cluster_setup_es<1>(), cluster_setup_es<2>(), cluster_setup_es<4>()});
+  return (uint32_t)eng.wide_cluster;
 }
 template <int ES>
 static cudaError_t launch_cluster_es(const P &p, uint32_t blocks, uint32_t fs, uint32_t max_rounds, cudaStream_t S) {
@@ -1014,14 +1011,11 @@ static uint32_t grid_setup_es(int device) {
   }
   return per > 0 ? (uint32_t)sms : 0u;
 }
-static uint32_t grid_blocks(int device, uint32_t es) {
-  static std::once_flag once[64];
-  static uint32_t blocks[64] = {};
-  if (device < 0 || device >= 64 || (es != 1 && es != 2 && es != 4)) return 0;
-  std::call_once(once[device], [device]() {
-    blocks[device] = std::min({grid_setup_es<1>(device), grid_setup_es<2>(device), grid_setup_es<4>(device)});
-  });
-  return blocks[device];
+static uint32_t grid_blocks(Engine &eng, int device, uint32_t es) {
+  if (es != 1 && es != 2 && es != 4) return 0;
+  if (eng.wide_grid < 0)
+    eng.wide_grid = (int)std::min({grid_setup_es<1>(device), grid_setup_es<2>(device), grid_setup_es<4>(device)});
+  return (uint32_t)eng.wide_grid;
 }
 template <int ES>
 static cudaError_t launch_rounds_es(P p, bool grid, uint32_t blocks, uint32_t fs, uint32_t max_rounds,
@@ -1205,8 +1199,10 @@ static geq_status solve_one_game(Engine &eng, int device, const GameInput &gi, c
   p.next = d_next;
   uint64_t rounds = 0;
   uint32_t *d_items = nullptr;  // the slots of a round that are computed again
-  const bool grid = n > WIDE_CLUSTER_POSITIONS && n <= WIDE_GRID_POSITIONS && grid_blocks(device, es) != 0u;
-  const uint32_t cluster = grid ? grid_blocks(device, es) : n <= WIDE_GRID_POSITIONS ? cluster_blocks(device, es) : 0u;
+  const bool grid = n > WIDE_CLUSTER_POSITIONS && n <= WIDE_GRID_POSITIONS && grid_blocks(eng, device, es) != 0u;
+  const uint32_t cluster = grid                       ? grid_blocks(eng, device, es)
+                           : n <= WIDE_GRID_POSITIONS ? cluster_blocks(eng, es)
+                                                      : 0u;
   const auto t_start = std::chrono::steady_clock::now();
   while (fsize) {
     bool first_try = true;  // of this round's slots
