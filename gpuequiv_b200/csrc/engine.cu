@@ -90,7 +90,7 @@ constexpr int SM_BM2 = 128;   // 128 words: second bitmap (own / old list)
 constexpr int SM_TMP = 256;   // 32 words: segment map / compaction
 constexpr int SM_PINC = 288;  // 32 words: predecessor counts (inclusive scan)
 constexpr int SM_PBEG = 320;  // 32 words: predecessor row starts
-constexpr int SM_WORDS = 352; // the lane path's W_* layout uses the same words at another time
+constexpr int SM_WORDS = 352; // (k_round's and the cluster kernels' W_* layout shares these words)
 // device error bits (Ctr::error)
 constexpr uint32_t DERR_LIST = 1u;     // a list longer than 2^24 - 1 energies
 constexpr uint32_t DERR_BOUNDS = 2u;   // checked build: index out of range
@@ -2998,11 +2998,9 @@ geq_status Engine::create(int device, std::unique_ptr<Engine> &out) {
   CU(cudaFuncSetAttribute(k_round<CodecStd, 2>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   CU(cudaFuncSetAttribute(k_round<CodecStd, 3>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   CU(cudaFuncSetAttribute(k_round<CodecStd, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  CU(cudaFuncSetAttribute(k_round<CodecStd, 5>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   CU(cudaFuncSetAttribute(k_round<CodecGen, 2>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   CU(cudaFuncSetAttribute(k_round<CodecGen, 3>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   CU(cudaFuncSetAttribute(k_round<CodecGen, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  CU(cudaFuncSetAttribute(k_round<CodecGen, 5>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   CU(cudaFuncSetAttribute(k_round_big<CodecStd>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   CU(cudaFuncSetAttribute(k_round_big<CodecGen>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   {
@@ -3557,14 +3555,17 @@ struct RoundKernel {
 };
 template <class Cd>
 static void round_kernels(const Engine &E, const KParams &kp, RoundKernel (&k)[4]) {
-  const uint32_t bps = std::min<uint32_t>(std::max<uint32_t>(E.tuning.blocks_per_sm, 2), 5);
+  // 5 runs as 4: the lanes' buffers leave room for four blocks.  (With buffers
+  // cut to fit five, 48 registers spill 150 bytes: 700 spectroscopy games 5.66
+  // ms, four blocks 5.11; the full buffers at four save 2 % on games of 10,000 to
+  // 30,000 positions.)
+  const uint32_t bps = std::min<uint32_t>(std::max<uint32_t>(E.tuning.blocks_per_sm, 2), 4);
   const unsigned long long nr = (kp.n_nodes + WARPS_PER_BLOCK * SPREAD_MIN - 1) / (WARPS_PER_BLOCK * SPREAD_MIN),
                            nb = (kp.n_nodes + WARPS_PER_BLOCK - 1) / WARPS_PER_BLOCK;
   auto clamp = [](unsigned long long n, unsigned long long most) {
     return dim3((unsigned)std::max<unsigned long long>(1, std::min(n, most)));
   };
-  k[0].f = bps == 2 ? (void *)k_round<Cd, 2> : bps == 3 ? (void *)k_round<Cd, 3> : bps == 4 ? (void *)k_round<Cd, 4>
-                                                                                           : (void *)k_round<Cd, 5>;
+  k[0].f = bps == 2 ? (void *)k_round<Cd, 2> : bps == 3 ? (void *)k_round<Cd, 3> : (void *)k_round<Cd, 4>;
   k[0].grid = clamp(nr, (unsigned long long)E.n_sms * bps);
   k[1].f = (void *)k_round_big<Cd>;
   k[1].grid = clamp(nb, (unsigned long long)E.n_sms * GEQ_BIG_BLOCKS_PER_SM);
