@@ -1198,6 +1198,7 @@ static geq_status solve_one_game(Engine &eng, int device, const GameInput &gi, c
   p.front = d_front;
   p.next = d_next;
   uint64_t rounds = 0;
+  uint64_t compactions = 0;
   uint32_t *d_items = nullptr;  // the slots of a round that are computed again
   const bool grid = n > WIDE_CLUSTER_POSITIONS && n <= WIDE_GRID_POSITIONS && grid_blocks(eng, device, es) != 0u;
   const uint32_t cluster = grid                       ? grid_blocks(eng, device, es)
@@ -1254,6 +1255,7 @@ static geq_status solve_one_game(Engine &eng, int device, const GameInput &gi, c
       first_try = true;
       if (h.arena_full) {
         // compact the committed lists into a larger arena and run the round again
+        compactions++;
         std::vector<unsigned long long> hd(n), noff(n);
         WCU(cudaMemcpyAsync(hd.data(), d_desc, n * 8ull, cudaMemcpyDeviceToHost, S));
         WCU(cudaStreamSynchronize(S));
@@ -1344,6 +1346,7 @@ static geq_status solve_one_game(Engine &eng, int device, const GameInput &gi, c
   sol.stats.positions_computed += h.positions;
   sol.stats.edges_relaxed += h.edges;
   sol.stats.algorithmic_bytes += h.bytes;
+  sol.stats.arena_compactions += compactions;
   sol.stats.kernel_launches += launches;
   sol.stats.device_ms += ms;
   (void)g_index;
