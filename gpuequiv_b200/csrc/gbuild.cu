@@ -1278,22 +1278,18 @@ static geq_status device_build(Engine &eng, int device, uint32_t n_jobs, const L
   const auto t1 = clk::now();
   db.b.reset(new gb::Builder<gb::DevBackend>(be));
   // start from the capacities the previous build of about as many start
-  // positions on this stream ended with (one hint for all sizes made a single
+  // positions on this engine ended with (one hint for all sizes made a single
   // query after a batch clear the batch's hash tables: equivalences() of a
-  // 40-state system 3.3 against 2.8 ms)
-  static std::mutex hint_mu;
-  static std::map<std::pair<void *, uint32_t>, gb::Builder<gb::DevBackend>::Caps> hints;
-  const std::pair<void *, uint32_t> hint_key((void *)be.s, 32u - lzcnt32(bin.n_starts));
-  {
-    std::lock_guard<std::mutex> g(hint_mu);
-    auto it = hints.find(hint_key);
-    if (it != hints.end()) db.b->hint = it->second;
-  }
+  // 40-state system 3.3 against 2.8 ms).  The capacities of one such size only
+  // grow: small single queries after a large one still clear its tables.  At
+  // most 32 sizes, and they go with the engine.
+  using Hints = std::map<uint32_t, gb::Builder<gb::DevBackend>::Caps>;
+  if (!eng.build_hints) eng.build_hints = std::make_shared<Hints>();
+  Hints &hints = *(Hints *)eng.build_hints.get();
+  const uint32_t hint_key = 32u - lzcnt32(bin.n_starts);
+  if (const auto it = hints.find(hint_key); it != hints.end()) db.b->hint = it->second;
   const int rc = db.b->run(bin, db.r);
-  if (rc == 0) {
-    std::lock_guard<std::mutex> g(hint_mu);
-    hints[hint_key] = db.b->used;
-  }
+  if (rc == 0) hints[hint_key] = db.b->used;
   db.upload_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
   db.build_ms = std::chrono::duration<double, std::milli>(clk::now() - t1).count();
   if (!be.ok()) return fail(GEQ_ERR_CUDA, "device game build: %s", cudaGetErrorString(be.err));

@@ -271,6 +271,7 @@ class Engine {
   // engine, not per process: the kernels' attributes belong to the CUDA
   // context and are gone when the device was reset between two engines.
   int build_cluster = -1, wide_cluster = -1, wide_grid = -1;
+  std::shared_ptr<void> build_hints;  // the device builder's capacities by size
   geq_tuning tuning{};
   int n_sms = 0;
   uint64_t total_mem = 0;
