@@ -407,7 +407,7 @@ geq_status geq_energy_game_run_batch(geq_context *ctx, uint32_t n_games, const g
     return GEQ_OK;
   }
   if (n_games == 1) {
-    // a small single game: one launch of the one-block solver
+    // a small single game: one launch (Engine::solve_small)
     std::unique_ptr<geq_solution> sol(new geq_solution());
     bool handled = false;
     if ((st = e->solve_small(in[0], *sol, handled))) return st;

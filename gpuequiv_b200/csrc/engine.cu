@@ -26,11 +26,11 @@
 //     (attackers first, each kind in position order).
 //   * Rounds are launched as CUDA graphs of several rounds each; the host
 //     reads one small counter block per graph launch to detect termination.
-//   * Uploads of up to 32,768 positions, and the rounds of uploads of up to a
-//     million whose frontier has become small, run inside one launch of a
-//     cluster of 16 blocks (k_rounds_cluster), a lone small game from upload
-//     to result (k_solve_static): their rounds are shorter than the launches
-//     of four kernels.
+//   * Uploads of up to 32,768 positions and 196,608 edges, and the rounds of
+//     uploads of up to a million positions whose frontier has become small, run
+//     inside one launch of a cluster of 16 blocks (k_rounds_cluster), a lone
+//     small game from upload to result (k_solve_static): their rounds are
+//     shorter than the launches of four kernels.
 //   * k_round spreads a small frontier over all its warps (lanes_solve: the
 //     positions of a warp worked on together), and long predecessor lists are
 //     cut into parts for k_round_big's warps (pushq).
@@ -1012,7 +1012,7 @@ __device__ Res solve_position(const WarpCtx &x, const Cd &cd, uint32_t v) {
 
 // ---- lane path: up to 32 positions per warp, one owner lane each ------------
 // Successor and update of edge k: one 8-byte load of the edge pair, or the
-// col / wt arrays where there are none (the one-block solver).
+// col / wt arrays where there are none (k_solve_static).
 __device__ __forceinline__ void load_edge(const KParams &p, Ctr *c, unsigned long long k, uint32_t &w, uint32_t &u) {
   if (p.cw) {
     const unsigned long long e = ld(p.cw, k, p.n_edges, c);
@@ -4956,7 +4956,7 @@ static geq_status static_scratch(int device, unsigned char *&out) {
   return GEQ_OK;
 }
 
-// Layout of a one-block solve (k_solve_static) inside one memory block:
+// Layout of a one-launch solve (k_solve_static) inside one memory block:
 // control block, the game, reverse CSR, descriptors, frontiers, result
 // offsets, 256-byte aligned, then the energy arena up to the block's end.
 struct BlockLayout {

@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(CLT, 1) k_assemble_cluster(View v, Out o, uint
 }
 
 // Signature refinement of a small batch (and the minimised systems) in one
-// launch: five barriers per iteration instead of eight launches and three
+// launch: six barriers per iteration instead of eight launches and three
 // fills, no read-back to learn whether it converged, and no iteration beyond
 // the one that shows it.
 __global__ void __launch_bounds__(CLT, 1) k_refine_cluster(const rf::Small a) {

@@ -241,7 +241,6 @@ class Refiner {
   ~Refiner() { release_all(); }
   // 0 ok; 1 out of memory / backend failure; 3 repeated fingerprint collisions
   int run(const gb::Input &in) {
-    small_ = false;
     if constexpr (gb::has_cluster<B>::value) {
       if (be_.cluster_refine_ok(in.NS, in.n_jobs)) {
         for (uint32_t attempt = 0; attempt < 4; attempt++) {
@@ -340,7 +339,6 @@ class Refiner {
   uint32_t hflags_[2] = {0, 0};
   const uint32_t *final_ = nullptr;
   Small sm_{};
-  bool small_ = false;
   static unsigned long long seed_of(uint32_t attempt) {
     return 0x13198a2e03707344ull + 0x9e3779b97f4a7c15ull * attempt;
   }
@@ -434,7 +432,6 @@ class Refiner {
     final_ = s.part[iterations & 1];
     final_isrep_ = s.isrep[(iterations - 1) & 1];
     final_rank_ = s.rank[(iterations - 1) & 1];
-    small_ = true;
     return 0;
   }
   uint32_t *final_isrep_ = nullptr, *final_rank_ = nullptr;
